@@ -198,12 +198,13 @@ TOTEM_API int totem_transmission_run(const TotemStemArgs *args, TotemStemOut *ou
  * counterpart in the reference, whose cal_p sums every atom at every pixel.
  *   TOTEM_TX_AUTO      the cheaper of the two by a cost model (default)
  *   TOTEM_TX_DIRECT    per-species sums over atoms at every pixel: O(atoms x pixels)
- *   TOTEM_TX_GRIDDING  Gaussian gridding onto a twice-finer grid and FFTs (a non-uniform FFT):
- *                      O(atoms + pixels log pixels), relative error ~1e-7; used where the axes
- *                      are uniform and the grid is a power of two from 64 to 4096, otherwise
- *                      DIRECT is used.
- * ``scratch_bytes`` bounds the gridding work memory taken during a build (0 = 1 GiB); at least
- * one species plane set (64 bytes per potential pixel) is always taken. */
+ *   TOTEM_TX_GRIDDING  gridding along y onto a twice-finer axis and FFTs (a non-uniform FFT), the
+ *                      x phases direct: O(atoms x width + pixels log pixels), relative error
+ *                      ~1e-7; used where the axes are uniform and the height is an edge of the
+ *                      fused transforms (64 to 4096, a power of two or a mixed-radix edge),
+ *                      otherwise DIRECT is used.
+ * ``scratch_bytes`` bounds the gridding work memory taken during a build (0 = 1 GiB); the arrays of
+ * one species of one slice (at most 64 bytes per potential pixel) are always taken. */
 #define TOTEM_TX_AUTO 0
 #define TOTEM_TX_DIRECT 1
 #define TOTEM_TX_GRIDDING 2

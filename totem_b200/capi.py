@@ -609,8 +609,8 @@ def set_slice_graphs(enable: bool):
 
 def set_tx_builder(mode: int, scratch_bytes: int = 0):
     """Process-wide transmission builder for separable grids (``totem_set_tx_builder``):
-    TX_AUTO (cost model), TX_DIRECT (sums over atoms at every pixel) or TX_GRIDDING (Gaussian
-    gridding + FFT where the axes are uniform); ``scratch_bytes`` bounds the gridding work memory
+    TX_AUTO (cost model), TX_DIRECT (sums over atoms at every pixel) or TX_GRIDDING (gridding
+    along y + FFT where the axes are uniform); ``scratch_bytes`` bounds the gridding work memory
     (0 = the library default)."""
     check(load().totem_set_tx_builder(int(mode), int(scratch_bytes)))
 

@@ -105,32 +105,58 @@ Status launch_tx_structure(const TxGrid& g, const AtomRowsDev& neutral, const At
 // species (no exponential per atom and pixel), then the form factor once per species and pixel.
 // Overwrites out.
 Status launch_tx_species(const TxGrid& g, const SpeciesSet& sp, float2* out, cudaStream_t st);
-// The same sums by Gaussian gridding (a type-1 non-uniform FFT) on uniform separable grids.
-// Work is grouped in jobs, one per (slice, kind, species) segment, ordered by slice; a batch
-// runs the jobs [j_lo, j_hi) in scratch memory and writes slices [s_lo, s_hi) (the last may be
-// partial, finished by the next batch).
+// The same sums by gridding along y (tx_grid.cuh) on separable grids with a uniform ky axis and a
+// height the fused transforms take.  Work is grouped in jobs, one per (slice, kind, species)
+// segment, ordered by slice; a batch runs the jobs [j_lo, j_hi) in scratch memory and writes slices
+// [s_lo, s_hi) (the last may be partial, finished by the next batch).
 struct GridPlanDev {
-  double dkx = 0, dky = 0;         // spacing of the kx / ky axes
-  double sx = 0, sy = 0;           // kx(p_w / 2), ky(p_h / 2): the shift folded into each atom's weight
-  const float2* ax = nullptr;      // [p_w][2]: Gaussian deconvolution x half-bin phase (parity 0, 1)
-  const float2* ay = nullptr;      // [p_h][2]
+  double dky = 0;                  // spacing of the ky axis
+  double sy = 0;                   // ky(p_h / 2): the shift folded into each atom's phase
+  int half = 0;                    // centred antisymmetric axes: S(-k) = conj S(k), columns kx >= 0 only
+  const float2* ay = nullptr;      // [p_h][2]: deconvolution x half-bin phase (parity 0, 1)
   const int4* jobs = nullptr;      // [jobs]: kind (SpeciesSet index), species, first atom, end atom
   const int* job_beg = nullptr;    // [slices + 1] first job of every slice
+  const int* atom_beg = nullptr;   // [jobs + 1] atoms of the jobs before
+};
+// Work memory of the gridding builder (grid_work lays it out): tables of all jobs of the build, and
+// the large arrays of one batch of jobs.
+struct GridWork {
+  int kmax = 0;                    // atoms of the largest job
+  int cols = 0, pitch = 0, half = 0;  // columns formed (p_w, or p_w / 2 + 1 when half), row pitch
+  // all jobs; a job's atoms start at GridPlanDev::atom_beg
+  float4* wgt = nullptr;           // [atoms][2]: the spreading weights of every group
+  int* bin = nullptr;              // [atoms]: first fine row of every atom (job order)
+  int* base = nullptr;             // [atoms]: first fine row of every group
+  int* order = nullptr;            // [atoms]: the job's atoms sorted by fine row
+  int* first = nullptr;            // [atoms + jobs]: first sorted atom of every group, then the atom count
+  int* ptr = nullptr;              // [jobs][2 p_h + 1]: first group of every fine row
+  int* groups = nullptr;           // [jobs]
+  unsigned char* used = nullptr;   // [jobs][2 p_h / 16]: a group spreads into this block of fine rows
+  // one batch
+  int ex_cols = 0;                 // columns of E held at a time (a multiple of 128, or pitch)
+  float2* ex = nullptr;            // [jobs][kmax][ex_cols]
+  float2* fine = nullptr;          // [jobs][2 p_h][pitch]
+  float2* s = nullptr;             // [jobs][p_h + 1][pitch]
 };
 struct GridBatch {
   int s_lo, s_hi, j_lo, j_hi;
 };
 std::vector<GridBatch> grid_batches(const std::vector<int>& job_beg, int jobs_per_batch);
-// Scratch of one job: four p_h x p_w planes of 16-byte points and a flag per fine row.
-inline size_t grid_job_bytes(int p_h, int p_w) { return (size_t)p_h * p_w * 64 + (size_t)p_h * 8; }
-// Overwrites out like launch_tx_species; ``scratch`` holds at least one job.  ``scratch_zero``:
-// the scratch is as an earlier call left it (otherwise it is cleared whole first).
+// Work memory: bytes of the tables of all jobs, and of one job's large arrays in a batch.
+struct GridBytes {
+  size_t tables, per_job;
+};
+GridBytes grid_bytes(int p_h, int p_w, int half, int kmax, int jobs, long long atoms);
+// Overwrites out like launch_tx_species; ``scratch`` holds the tables and at least one job's arrays.
+// With ``finish`` (the transmission's fused FFT takes the grid and nothing is to be added to V) out
+// receives T = exp(i sig V) of every slice and *finished is set, unless a slice has more jobs than a
+// batch holds.
 Status launch_tx_gridding(const TxGrid& g, const SpeciesSet& sp, const GridPlanDev& gp,
-                          const std::vector<int>& job_beg, const std::vector<int4>& jobs, const float2* tw_w,
-                          const float2* tw_h, void* scratch, size_t scratch_bytes, bool scratch_zero, float2* out,
-                          cudaStream_t st, int* launches);
-// Per-axis factors of the gridding builder for an axis of n points: [c][parity] = the inverse
-// of the spreading Gaussian's transform (normalised) times exp(-i pi k parity / n), k = c - n/2.
+                          const std::vector<int>& job_beg, int kmax, long long atoms, const float2* tw_w,
+                          const float2* tw_h, void* scratch, size_t scratch_bytes, bool finish, float sig, float2* out,
+                          cudaStream_t st, int* launches, bool* finished);
+// Factors of the gridding builder along y for an axis of n points: [r][parity] = the inverse of
+// the spreading kernel's transform times exp(-i pi k parity / n), k = r - n/2.
 std::vector<float2> grid_deconvolution(int n);
 // Process-wide builder choice for separable grids (TOTEM_TX_*) and gridding scratch bytes.
 int tx_builder_mode();
@@ -145,10 +171,9 @@ Status launch_tx_fft_exp(float2* data, int slices, int p_h, int p_w, float sigma
 // Element-wise (-1)^(r+c) and exp for the cuFFT builder.
 Status launch_sign_exp(float2* data, long total, int p_h, int p_w, float sigma_scaled, cudaStream_t st);
 
-// Grid edges of the fused transmission FFT (powers of two 64..4096 and the mixed-radix edges of
-// TOTEM_MR_WINDOWS), and of the gridding builder (powers of two 64..4096).
+// Grid edges of the fused transmission FFT and heights of the gridding builder: powers of two
+// 64..4096 and the mixed-radix edges of TOTEM_MR_WINDOWS.
 bool fused_fft_size_ok(int n);
-bool gridding_size_ok(int n);
 // Whether the fused transmission FFT takes a p_h x p_w grid of ``slices`` slices: both edges
 // fused_fft_size_ok, the rows of all slices whole row tiles of p_w and the width whole column
 // tiles of p_h.
@@ -280,6 +305,11 @@ struct WindowOps {
   // the transmission's inverse FFT: rows of length n, then columns of length n with the sign and exp
   Status (*tx_rows_inv)(float2* data, long nrows, const float2* tw, cudaStream_t st);
   Status (*tx_cols_exp)(float2* data, int slices, int p_w, const float2* tw, float sig, cudaStream_t st);
+  // the gridding builder at height n (grid_cols, grid_cols_inv) and its rows of length n (rows_exp)
+  Status (*grid_cols)(const GridWork& w, int job0, int jobs, const float2* ay, const float2* tw, cudaStream_t st);
+  Status (*grid_cols_inv)(const TxGrid& g, const SpeciesSet& sp, const GridPlanDev& gp, const GridWork& w, int s_lo,
+                          int s_hi, int j_lo, float2* out, const float2* tw, cudaStream_t st);
+  Status (*tx_rows_exp)(float2* data, long nrows, const float2* tw, float sig, cudaStream_t st);
 };
 const WindowOps* radix_window_ops(int n);
 

@@ -492,6 +492,8 @@ Status totem_session::build_transmission(int path, int* launches) {
   g.cim_len = cim_len;
   const auto vcn = rows_cn.view(cim_len > 0 && n_corr > 0, false, 3);
   const auto vci = rows_ci.view(cim_len > 0 && n_corr_i > 0, false, 6);
+  const float sig = (float)(sigma / 1000.0);
+  bool finished = false;  // T already holds exp(i sigma V) (the gridding builder's own transforms)
   if (separable) {
     totem::SpeciesSet set;
     set.k[0] = species_n.view(n_rows > 0, has_abs_n, ncoef_n);
@@ -501,33 +503,36 @@ Status totem_session::build_transmission(int path, int* launches) {
       set.k[3] = species_ci.view(cim_len > 0 && n_corr_i > 0, false, 6);
     }
     const int mode = totem::tx_builder_mode();
-    if (grid_ok && (mode == TOTEM_TX_GRIDDING || (mode == TOTEM_TX_AUTO && gridding_cheaper()))) {
-      // jobs per batch from the budget for their planes (64 bytes per pixel); the row flags on top
-      const size_t jobs = std::max<size_t>(grid_jobs_h.size(), 1);
-      const size_t per = std::min(totem::tx_gridding_scratch() / ((size_t)p_h * p_w * 64), jobs);
-      const size_t bytes = std::max<size_t>(1, per) * totem::grid_job_bytes(p_h, p_w);
-      // the state the kernels leave the scratch in depends on the row layout and the batch size
-      const long long layout = ((long long)p_h << 40) | ((long long)p_w << 20) | (long long)std::max<size_t>(1, per);
-      if (bytes > grid_scratch.cap || layout != grid_scratch_layout) grid_scratch_zero = false;
-      TOTEM_TRY(grid_scratch.ensure(bytes));
-      grid_scratch_layout = layout;
-      totem::GridPlanDev gp;
-      gp.dkx = grid_dkx; gp.dky = grid_dky; gp.sx = grid_sx; gp.sy = grid_sy;
-      gp.ax = grid_ax.as<float2>(); gp.ay = grid_ay.as<float2>();
-      gp.jobs = grid_jobs.as<int4>(); gp.job_beg = grid_job_beg.as<int>();
-      const bool was_zero = grid_scratch_zero;
-      grid_scratch_zero = false;  // until every batch has been enqueued
-      ran_tx_builder = TOTEM_TX_GRIDDING;
-      TOTEM_TRY(totem::launch_tx_gridding(g, set, gp, grid_job_beg_h, grid_jobs_h, tw_pw.as<float2>(),
-                                          tw_ph.as<float2>(), grid_scratch.p, bytes, was_zero, T.as<float2>(), stream,
-                                          launches));
-      grid_scratch_zero = true;  // left as the next build expects it (in stream order)
-      // work memory of the build only: returned at once to a server's pool (stream-ordered and
-      // cheap); a plain session keeps it, cleared, for its next build (cudaFree would synchronise)
-      if (grid_scratch.pool) {
-        grid_scratch.release();
-        grid_scratch_zero = false;
+    bool gridding = grid_ok && (mode == TOTEM_TX_GRIDDING || (mode == TOTEM_TX_AUTO && gridding_cheaper()));
+    size_t bytes = 0;
+    if (gridding) {
+      // jobs per batch from the budget for their work memory, at least one; a device that has no
+      // room for it takes the direct sums, unless gridding was asked for
+      const totem::GridBytes need = totem::grid_bytes(p_h, p_w, grid_half, grid_kmax, grid_job_beg_h.back(), grid_atoms);
+      const size_t room = std::max(totem::tx_gridding_scratch(), need.tables + need.per_job) - need.tables;
+      const size_t jobs = std::max(grid_job_beg_h.back(), 1);
+      bytes = need.tables + need.per_job * std::min(room / need.per_job, jobs);
+      const Status st = grid_scratch.ensure(bytes);
+      if (!st.ok()) {
+        if (mode == TOTEM_TX_GRIDDING || st.code != TOTEM_ERR_OOM) return st;
+        cudaGetLastError();  // the failed allocation's error
+        gridding = false;
       }
+    }
+    if (gridding) {
+      totem::GridPlanDev gp;
+      gp.dky = grid_dky; gp.sy = grid_sy; gp.half = grid_half;
+      gp.ay = grid_ay.as<float2>();
+      gp.jobs = grid_jobs.as<int4>(); gp.job_beg = grid_job_beg.as<int>();
+      gp.atom_beg = grid_atom_beg.as<int>();
+      ran_tx_builder = TOTEM_TX_GRIDDING;
+      const bool finish = path != TOTEM_PATH_PLAIN && fft_fused && (corr_by_species || !(vcn.beg || vci.beg));
+      TOTEM_TRY(totem::launch_tx_gridding(g, set, gp, grid_job_beg_h, grid_kmax, grid_atoms, tw_pw.as<float2>(),
+                                          tw_ph.as<float2>(), grid_scratch.p, bytes, finish, sig, T.as<float2>(),
+                                          stream, launches, &finished));
+      // work memory of the build only: returned at once to a server's pool (stream-ordered and
+      // cheap); a plain session keeps it for its next build (cudaFree would synchronise)
+      if (grid_scratch.pool) grid_scratch.release();
     } else {
       ran_tx_builder = TOTEM_TX_DIRECT;
       TOTEM_TRY(totem::launch_tx_species(g, set, T.as<float2>(), stream));
@@ -545,8 +550,9 @@ Status totem_session::build_transmission(int path, int* launches) {
     TOTEM_TRY(totem::launch_tx_structure(g, vn, vi, vcn, vci, T.as<float2>(), stream));
     ++*launches;
   }
-  const float sig = (float)(sigma / 1000.0);
-  if (path != TOTEM_PATH_PLAIN && fft_fused) {
+  if (finished) {
+    ran_tx_fft = TOTEM_PATH_FUSED;
+  } else if (path != TOTEM_PATH_PLAIN && fft_fused) {
     ran_tx_fft = TOTEM_PATH_FUSED;
     TOTEM_TRY(totem::launch_tx_fft_exp(T.as<float2>(), slices, p_h, p_w, sig, tw_pw.as<float2>(),
                                        tw_ph.as<float2>(), stream));
@@ -565,15 +571,15 @@ Status totem_session::build_transmission(int path, int* launches) {
 }
 
 // Uniform separable axes, kx(c) = kx0 + c dkx and ky(r) = ky0 + r dky (the reference's
-// meshgrid of (-P/2 : P/2-1) / (P dx), ToTEM_submit_v1.m:1534-1538), on power-of-two grids admit
-// the gridding builder.  Its job table holds one job per species segment of every slice
-// (neutral, ionic, then the correction kinds), in slice order.
+// meshgrid of (-P/2 : P/2-1) / (P dx), ToTEM_submit_v1.m:1534-1538), on a grid whose height the
+// fused transforms take admit the gridding builder.  Its job table holds one job per species segment
+// of every slice (neutral, ionic, then the correction kinds), in slice order.
 Status totem_session::plan_gridding(const TotemStemArgs* a, const totem::SpeciesHost* const (&kinds)[4]) {
   grid_ok = false;
   grid_job_beg_h.clear();
-  grid_jobs_h.clear();
   grid_atoms = 0;
-  if (!totem::gridding_size_ok(p_h) || !totem::gridding_size_ok(p_w) || slices <= 0) return Status::Ok();
+  grid_kmax = 1;
+  if (!totem::fused_fft_size_ok(p_h) || slices <= 0) return Status::Ok();
   auto uniform = [](const double* v, int n, long stride, double* d) {
     *d = (v[(long)(n - 1) * stride] - v[0]) / (n - 1);
     if (!std::isfinite(*d) || *d == 0.0) return false;
@@ -583,44 +589,49 @@ Status totem_session::plan_gridding(const TotemStemArgs* a, const totem::Species
   };
   double dkx = 0, dky = 0;
   if (!uniform(a->kx, p_w, 1, &dkx) || !uniform(a->ky, p_h, p_w, &dky)) return Status::Ok();
-  grid_dkx = dkx;
   grid_dky = dky;
-  grid_sx = a->kx[0] + dkx * (p_w / 2);
-  grid_sy = a->ky[0] + dky * (p_h / 2);
+  grid_sy = a->ky[(size_t)(p_h / 2) * p_w];
+  // S(-k) = conj S(k) column by column: kx antisymmetric about its middle column, ky centred
+  grid_half = grid_sy == 0.0 && a->kx[p_w / 2] == 0.0;
+  for (int c = 1; c < p_w / 2 && grid_half; ++c) grid_half = a->kx[p_w / 2 - c] == -a->kx[p_w / 2 + c];
+  std::vector<int4> jobs;
+  std::vector<int> atom_beg(1, 0);
   grid_job_beg_h.assign(slices + 1, 0);
   for (int s = 0; s < slices; ++s) {
     for (int kind = 0; kind < 4; ++kind) {
       const totem::SpeciesHost& sp = *kinds[kind];
       if ((int)sp.seg_beg.size() != slices + 1) continue;
       for (int q = sp.seg_beg[s]; q < sp.seg_beg[s + 1]; ++q) {
-        grid_jobs_h.push_back(make_int4(kind, sp.seg[3 * q], sp.seg[3 * q + 1], sp.seg[3 * q + 2]));
-        grid_atoms += sp.seg[3 * q + 2] - sp.seg[3 * q + 1];
+        const int atoms = sp.seg[3 * q + 2] - sp.seg[3 * q + 1];
+        jobs.push_back(make_int4(kind, sp.seg[3 * q], sp.seg[3 * q + 1], sp.seg[3 * q + 2]));
+        grid_atoms += atoms;
+        atom_beg.push_back((int)grid_atoms);
+        grid_kmax = std::max(grid_kmax, atoms);
       }
     }
-    grid_job_beg_h[s + 1] = (int)grid_jobs_h.size();
+    grid_job_beg_h[s + 1] = (int)jobs.size();
   }
   cudaStream_t st = stream;
-  TOTEM_TRY(upload(grid_jobs, grid_jobs_h, st));
+  TOTEM_TRY(upload(grid_jobs, jobs, st));
   TOTEM_TRY(upload(grid_job_beg, grid_job_beg_h, st));
-  TOTEM_TRY(upload(grid_ax, totem::grid_deconvolution(p_w), st));
+  TOTEM_TRY(upload(grid_atom_beg, atom_beg, st));
   TOTEM_TRY(upload(grid_ay, totem::grid_deconvolution(p_h), st));
   grid_ok = true;
   return Status::Ok();
 }
 
-// Cost model of the two separable builders, measured on B200 (SrTiO3 supercells filling the
-// grid, 20 slices): the direct sums take ~0.29 ps per atom and pixel; gridding takes per job
-// (species and slice) and pixel 29 ps at 1024^2, 35 ps at 2048^2 and 44 ps at 4096^2 (the
-// long column transforms run below bandwidth), plus ~20 us of launches per batch.
+// Cost model of the two separable builders, measured on B200 (SrTiO3 blocks of 1 to 64 unit cells
+// and grid-filling ones, 6 and 40 slices): the direct sums take 0.29 ps per atom and pixel.  Gridding
+// hardly depends on the atoms; against the direct sums without any atom it takes under 1 ps more
+// per job (species and slice) and pixel where the columns are two-stage transforms (powers of two up
+// to 1024), up to 4 ps at other heights, and ~12 us for its launches.  So it pays from 4 or 14 atoms
+// per job on: 40 slices at 1024^2 with 4 / 16 / 64 / 256 atoms per job, direct against gridding, 0.97 /
+// 1.29 / 2.71 / 8.46 against 0.90 / 0.92 / 1.01 / 1.13 ms; at 1280^2 1.71 / 2.21 / 4.41 / 20.1 (400)
+// against 2.26 / 2.29 / 2.35 / 2.66 ms.
 bool totem_session::gridding_cheaper() const {
-  const double plane = (double)p_h * p_w;
-  const double jobs = (double)grid_jobs_h.size();
-  const int edge = std::max(p_h, p_w);
-  const double per_px = edge <= 1024 ? 2.9e-11 : (edge <= 2048 ? 3.5e-11 : 4.4e-11);
-  const double per_batch = std::max(1.0, std::floor((double)totem::tx_gridding_scratch() / (plane * 64.0)));
-  const double direct = 2.9e-13 * (double)grid_atoms * plane;
-  const double gridding = per_px * jobs * plane + 2e-5 * (std::ceil(jobs / per_batch) + 1);
-  return gridding < direct;
+  const double plane = (double)p_h * p_w, jobs = (double)grid_job_beg_h.back();
+  const double per_px = (p_h <= 1024 && is_pow2(p_h)) ? 1e-12 : 4e-12;
+  return per_px * jobs * plane + 1.2e-5 < 2.9e-13 * (double)grid_atoms * plane;
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -3,7 +3,7 @@
 // groups.cu; mixed-radix windows: windows_mixed_*.cu).
 #pragma once
 #include "hrtem_kernels.cuh"
-#include "tx_fft.cuh"
+#include "tx_grid.cuh"
 #include "slice_tiles.cuh"
 
 namespace totem {
@@ -233,7 +233,10 @@ const WindowOps* window_ops() {
                              RowCfg<N>::G,
                              GridColCfg<N>::G,
                              &rows_inv<N>,
-                             &cols_exp<N>};
+                             &cols_exp<N>,
+                             &grid_cols<N>,
+                             &grid_cols_inv<N>,
+                             &rows_exp<N>};
   return &ops;
 }
 

@@ -168,15 +168,14 @@ struct totem_session {
   totem::SpeciesRowsDev species_cn, species_ci;  // the correction rows by species (separable grids)
   // correction rows by species (few distinct rows per slice), or by the per-atom kernel on top
   bool corr_by_species = true;
-  // gridding builder (uniform separable axes): job table, deconvolution tables, work memory
+  // gridding builder (uniform separable axes): job table, deconvolution table, work memory
   bool grid_ok = false;
-  bool grid_scratch_zero = false;  // grid_scratch is as the last gridding build left it, for
-  long long grid_scratch_layout = -1;  // that build's grid and jobs per batch
-  double grid_dkx = 0, grid_dky = 0, grid_sx = 0, grid_sy = 0;
+  double grid_dky = 0, grid_sy = 0;
+  int grid_half = 0;  // centred antisymmetric axes (GridPlanDev::half)
+  int grid_kmax = 1;  // atoms of the largest job
   long long grid_atoms = 0;
   std::vector<int> grid_job_beg_h;
-  std::vector<int4> grid_jobs_h;
-  totem::DevBuf grid_jobs, grid_job_beg, grid_ax, grid_ay, grid_scratch;
+  totem::DevBuf grid_jobs, grid_job_beg, grid_atom_beg, grid_ay, grid_scratch;
   totem::DevBuf kx_axis, ky_axis, kx, ky, s2, aper_true, cim;
   // work buffers and results
   totem::DevBuf T, psi, part, acc, out_result, out_mid;
@@ -225,7 +224,7 @@ struct totem_session {
     for (totem::DevBuf* b : {&probe, &prop, &mask_mid, &mask_exit, &tw_n, &tw_pw, &tw_ph, &gfsf_d, &kx_axis, &ky_axis,
                              &kx, &ky, &s2, &aper_true, &cim, &T, &psi, &part, &acc, &out_result, &out_mid,
                              &ev_slice, &Tb, &hr_wave, &hr_prop, &hr_tf, &hr_w, &hr_work, &hr_exit, &hr_img, &grid_jobs,
-                             &grid_job_beg, &grid_ax, &grid_ay, &grid_scratch})
+                             &grid_job_beg, &grid_atom_beg, &grid_ay, &grid_scratch})
       f(*b);
     for (totem::RowsDev* r : {&rows_n, &rows_i, &rows_cn, &rows_ci})
       for (totem::DevBuf* b : {&r->pos, &r->coef, &r->absorp, &r->beg}) f(*b);

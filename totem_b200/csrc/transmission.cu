@@ -19,7 +19,7 @@
 
 #include "common.cuh"
 #include "fft.cuh"
-#include "tx_fft.cuh"
+#include "tx_grid.cuh"
 
 namespace totem {
 
@@ -30,74 +30,6 @@ constexpr int TX_PR = 4;       // rows per thread
 constexpr int TX_TR = 32;      // tile rows (8 warps x 4)
 constexpr int TX_CH = 32;      // atoms staged per chunk
 constexpr int TX_MAXC = 24;    // widest coefficient block (ionic Lobato row without x, y)
-
-__device__ __forceinline__ float peng5(const float* c, float s2) {
-  float f = 0.f;
-#pragma unroll
-  for (int i = 0; i < 5; ++i) f = fmaf(c[2 * i], __expf(-c[2 * i + 1] * s2), f);
-  return f;
-}
-
-__device__ __forceinline__ float lobato5(const float* c, float g2) {
-  float f = 0.f;
-#pragma unroll
-  for (int i = 0; i < 5; ++i) {
-    const float b = c[2 * i + 1];
-    const float d = fmaf(b, g2, 1.f);
-    f = fmaf(c[2 * i], __fdividef(fmaf(b, g2, 2.f), d * d), f);
-  }
-  return f;
-}
-
-// Form factor of one neutral (kind 0) or ionic (kind 1) coefficient row at s^2: real part fr
-// (Peng: occ * sum a_i exp(-b_i s^2); Lobato: occ * sum a_i (2 + b_i g^2) / (1 + b_i g^2)^2 *
-// exp(-B s^2), g^2 = 4 s^2; ionic rows mix the ion and atom sums by their fractions) and the
-// absorptive imaginary part fi (occ * Peng sum of the absorptive row, or 0).
-__device__ __forceinline__ void row_form(int kind, int lobato, const float* cf, const float* absorp, float s2,
-                                         float& fr, float& fi) {
-  if (kind == 0) {
-    if (lobato) fr = cf[0] * lobato5(cf + 1, 4.f * s2) * __expf(-cf[11] * s2);
-    else fr = cf[0] * peng5(cf + 1, s2);
-  } else {
-    if (lobato)
-      fr = cf[0] * (cf[1] * lobato5(cf + 2, 4.f * s2) + cf[12] * lobato5(cf + 13, 4.f * s2)) * __expf(-cf[23] * s2);
-    else fr = cf[0] * (cf[1] * peng5(cf + 2, s2) + cf[12] * peng5(cf + 13, s2));
-  }
-  fi = absorp != nullptr ? cf[0] * peng5(absorp, s2) : 0.f;
-}
-
-// Form factor of species ``sp`` of kind ``kind`` (SpeciesSet) at pixel ``pix`` (s^2 = s2):
-// kinds 0 / 1 as row_form; the Peng-extended correction kinds 2 / 3
-// (cuda_source_peng_and_corr.cu:587-779, GetPotential4AllSlice_multicore_lotabo_peng_corr.m:13-60)
-// amplitude * exp(-B s^2) * the correction plane(s) at the pixel (planes numbered from 1).
-__device__ __forceinline__ void species_form(int kind, const TxGrid& g, const SpeciesDev& d, int sp, float s2,
-                                             long pix, float& fr, float& fi) {
-  const float* cf = d.coef + (long)sp * d.ncoef;
-  if (kind <= 1) {
-    row_form(kind, g.lobato, cf, d.absorp != nullptr ? d.absorp + (long)sp * 10 : nullptr, s2, fr, fi);
-    return;
-  }
-  const long plane = (long)g.p_h * g.p_w;
-  float m = 0.f;
-  if (kind == 2) {
-    const int idx = (int)cf[2] - 1;
-    if (idx >= 0 && idx < g.cim_len) m = g.cim[idx * plane + pix];
-  } else {
-    const int i1 = (int)cf[3] - 1, i2 = (int)cf[5] - 1;
-    if (i1 >= 0 && i1 < g.cim_len) m = fmaf(cf[2], g.cim[i1 * plane + pix], m);
-    if (i2 >= 0 && i2 < g.cim_len) m = fmaf(cf[4], g.cim[i2 * plane + pix], m);
-  }
-  fr = cf[1] * m * __expf(-cf[0] * s2);
-  fi = 0.f;
-}
-
-// exp(-2 pi i t) for t given in FP64, reduced to [0, 1) before the FP32 evaluation.
-__device__ __forceinline__ float2 phase_of(double t) {
-  const double fr = t - floor(t);
-  float s, c;
-  sincospif(2.f * (float)fr, &s, &c);
-  return make_float2(c, -s);
-}
 
 struct TxSmem {
   double pos[TX_CH][2];
@@ -308,189 +240,264 @@ __global__ void __launch_bounds__(256, 2) k_tx_species(TxGrid g, SpeciesSet spse
 }
 
 // ---------------------------------------------------------------------------------------------
-// By species through Gaussian gridding (a type-1 non-uniform FFT), for uniform separable grids
-// kx(c) = kx0 + c dkx, ky(r) = ky0 + r dky.  With kx' = c - p_w/2, ky' = r - p_h/2,
-//   S(r, c) = sum_a w_a exp(-i (kx' tx_a + ky' ty_a)),
-//   tx_a = 2 pi frac(dkx x_a), ty_a = 2 pi frac(dky y_a),
-//   w_a = exp(-2 pi i (kx(p_w/2) x_a + ky(p_h/2) y_a))   (1 on centred grids).
-// Each atom is spread with a periodic Gaussian exp(-d^2 / (4 tau)) onto a grid twice as fine as
-// the potential (GR_W x GR_W points), the fine grid is transformed, and the Gaussian's transform
-// sqrt(pi / tau) exp(-k^2 tau) is divided out: Greengard & Lee, "Accelerating the nonuniform
-// fast Fourier transform", SIAM Review 46 (2004) 443-454, with oversampling R = 2, half-width
-// M_sp = 7 and tau = pi M_sp / (P^2 R (R - 1/2)).  The relative L2 error of S is ~1e-7 (below
-// the FP32 sums) whatever the atom count; the cost is O(atoms + P^2 log P) per species and
-// slice instead of O(atoms P^2).
-//
-// The 2P x 2P fine grid is held as four P x P planes by the parity of its indices, plane
-// (ey, ex) = points (2 qy + ey, 2 qx + ex), so its transform is four P x P FFTs and a half-bin
-// phase: F(k) = sum_{ey, ex} exp(-i pi (ky ey / p_h + kx ex / p_w)) FFT(plane_{ey,ex})[k mod P].
-// The x half of that sum is taken right after the row transforms (the rows of parity ex = 0
-// and 1 of a fine row pair share a CTA), together with the x deconvolution, so two planes per
-// job, ey = 0 and 1, go through the column transforms and the combine.
-// Atoms are added in 32.32 fixed point (64-bit integer atomics), so the grid, and everything
-// after it, is bit-reproducible whatever order the atomics land in.  The row pass writes its
-// complex64 output in place into the ex = 0 row (the first half of its 16-byte-per-point
-// storage), so the planes keep a pitch of 2 p_w complex64 values from then on.
+// Gridding (tx_grid.cuh): the kernels that do not depend on the transform length.
 // ---------------------------------------------------------------------------------------------
-constexpr int GR_MSP = 7;
-constexpr int GR_W = 2 * GR_MSP;
-constexpr float GR_FIX = 4294967296.f;         // 2^32
-constexpr float GR_UNFIX = 1.f / 4294967296.f;
+constexpr int GR_T = 256;
 
-__global__ void __launch_bounds__(256) k_grid_spread(GridPlanDev gp, int p_h, int p_w, SpeciesSet spset, int job0,
-                                                     unsigned long long* __restrict__ grid,
-                                                     unsigned* __restrict__ row_used) {
-  const int4 jb = gp.jobs[job0 + blockIdx.y];  // kind, species, first atom, end atom
-  const double* pos = spset.k[jb.x & 3].pos;
-  const long plane = (long)p_h * p_w;
-  unsigned long long* base = grid + (long)blockIdx.y * 8 * plane;  // 4 planes of (re, im) pairs
-  const int total = (jb.w - jb.z) * GR_W;
-  // h^2 / (4 tau) for the fine-grid spacing h = 2 pi / (2P): pi (R - 1/2) / (R M_sp)
-  const float kappa = 3.f * 3.14159265358979f / (4.f * GR_MSP);
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    const int q = t / GR_W, jy = t - q * GR_W;
-    const int a = jb.z + q;
-    const double x = pos[2L * a], y = pos[2L * a + 1];
-    const double fx = gp.dkx * x, fy = gp.dky * y;
-    const double u = (fx - floor(fx)) * (2.0 * p_w), v = (fy - floor(fy)) * (2.0 * p_h);
-    const double fu = floor(u), fv = floor(v);
-    const float du = (float)(u - fu), dv = (float)(v - fv);
-    const float2 w = phase_of(gp.sx * x + gp.sy * y);
-    const int my = ((int)fv + jy - (GR_MSP - 1)) & (2 * p_h - 1);
-    row_used[(long)blockIdx.y * 2 * p_h + my] = 1u;  // the row pass skips fine rows nobody touched
-    const float ey = (float)(jy - (GR_MSP - 1)) - dv;
-    unsigned long long* row = base + (long)(my & 1) * 4 * plane + (long)(my >> 1) * 2 * p_w;
-#pragma unroll 2
-    for (int jx = 0; jx < GR_W; ++jx) {
-      const int mx = ((int)fu + jx - (GR_MSP - 1)) & (2 * p_w - 1);
-      const float ex = (float)(jx - (GR_MSP - 1)) - du;
-      const float gw = __expf(-kappa * fmaf(ex, ex, ey * ey)) * GR_FIX;
-      unsigned long long* dst = row + (long)(mx & 1) * 2 * plane + 2 * (mx >> 1);
-      atomicAdd(dst, (unsigned long long)__float2ll_rn(w.x * gw));
-      atomicAdd(dst + 1, (unsigned long long)__float2ll_rn(w.y * gw));
+// Kaiser-Bessel shape parameter for GR_W points at oversampling 2, and I0 by its power series
+// (arguments up to 18.7; the terms left out are below 1e-17 of the sum).
+constexpr double GR_BETA = 18.638814;  // pi sqrt((GR_W / 2)^2 (3 / 2)^2 - 0.8)
+__host__ __device__ inline double bessel_i0(double z) {
+  const double q = 0.25 * z * z;
+  double t = 1.0, s = 1.0;
+#pragma unroll
+  for (int k = 1; k <= 48; ++k) {
+    t *= q * (1.0 / ((double)k * k));
+    s += t;
+  }
+  return s;
+}
+
+// Exclusive prefix sum of cnt[0 .. n) in shared memory, in place; returns the total.
+__device__ int block_exclusive_scan(int* cnt, int n, int* warp_sum) {
+  const int per = (n + GR_T - 1) / GR_T, lo = min(n, (int)threadIdx.x * per), hi = min(n, lo + per);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  __syncthreads();
+  int s = 0;
+  for (int i = lo; i < hi; ++i) s += cnt[i];
+  int x = s;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) warp_sum[wid] = x;
+  __syncthreads();
+  int before = x - s, total = 0;
+  for (int i = 0; i < GR_T / 32; ++i) {
+    if (i < wid) before += warp_sum[i];
+    total += warp_sum[i];
+  }
+  for (int i = lo; i < hi; ++i) {
+    const int c = cnt[i];
+    cnt[i] = before;
+    before += c;
+  }
+  __syncthreads();
+  return total;
+}
+
+// Fine-grid place of an atom: v in [0, 2 p_h], first row b = ceil(v - GR_W / 2) mod 2 p_h.
+__device__ __forceinline__ double fine_row(double y, double dky, int nf) {
+  const double t = dky * y;
+  return (t - floor(t)) * nf;
+}
+__device__ __forceinline__ int first_row(double v, int nf) {
+  const int b = (int)ceil(v - GR_W / 2);
+  return min(max(b < 0 ? b + nf : b, 0), nf - 1);
+}
+
+// One CTA per job: counting sort of its atoms by first fine row (stable: one warp places 32 atoms
+// at a time in order, so the result does not depend on timing), groups of adjacent atoms with the
+// same y, the first group of every fine row, and the blocks of fine rows a group reaches.
+__global__ void __launch_bounds__(GR_T) k_grid_sort(GridPlanDev gp, SpeciesSet spset, int p_h, GridWork w) {
+  extern __shared__ int cnt[];  // [2 p_h + 1]
+  __shared__ int warp_sum[GR_T / 32];
+  const int nf = 2 * p_h, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int4 jb = gp.jobs[blockIdx.x];
+  const int K = jb.w - jb.z;
+  const double* pos = spset.k[jb.x & 3].pos + 2L * jb.z;
+  const int at0 = gp.atom_beg[blockIdx.x];
+  int* bin = w.bin + at0;
+  int* base = w.base + at0;
+  int* order = w.order + at0;
+  int* first = w.first + at0 + blockIdx.x;
+  int* ptr = w.ptr + (long)blockIdx.x * (nf + 1);
+  unsigned char* used = w.used + (long)blockIdx.x * (nf / GR_ROWS);
+  for (int i = tid; i < nf; i += GR_T) cnt[i] = 0;
+  __syncthreads();
+  for (int a = tid; a < K; a += GR_T) {
+    const int b = first_row(fine_row(pos[2 * a + 1], gp.dky, nf), nf);
+    bin[a] = b;
+    atomicAdd(&cnt[b], 1);
+  }
+  block_exclusive_scan(cnt, nf, warp_sum);  // its barriers make bin visible to the CTA
+  if (wid == 0) {
+    constexpr int AHEAD = 4;  // chunks whose bins are loaded ahead of their placing
+    int nb[AHEAD];
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k) nb[k] = 32 * k + lane < K ? bin[32 * k + lane] : -1;
+    for (int a0 = 0; a0 < K; a0 += 32 * AHEAD) {
+#pragma unroll
+      for (int k = 0; k < AHEAD; ++k) {
+        const int a = a0 + 32 * k + lane, b = nb[k];
+        nb[k] = a + 32 * AHEAD < K ? bin[a + 32 * AHEAD] : -1;
+        const unsigned peers = __match_any_sync(0xffffffffu, b);  // lanes past the end: b = -1
+        const int at = b >= 0 ? cnt[b] : 0;
+        __syncwarp();
+        if (b >= 0) {
+          if (lane == __ffs(peers) - 1) cnt[b] = at + __popc(peers);
+          order[at + __popc(peers & ((1u << lane) - 1u))] = a;
+        }
+        __syncwarp();
+      }
+    }
+  }
+  __syncthreads();  // the whole CTA sees the sorted order
+  for (int i = tid; i < nf; i += GR_T) cnt[i] = 0;
+  int groups = 0;  // groups before the chunk
+  for (int i0 = 0; i0 < K; i0 += GR_T) {
+    const int i = i0 + tid;
+    bool head = false;
+    int row = 0;
+    if (i < K) {
+      const int a = order[i];
+      row = bin[a];
+      head = i == 0 || !(pos[2 * order[i - 1] + 1] == pos[2 * a + 1]);
+    }
+    const unsigned heads = __ballot_sync(0xffffffffu, head);
+    __syncthreads();  // warp_sum of the previous chunk is read
+    if (lane == 0) warp_sum[wid] = __popc(heads);
+    __syncthreads();
+    int gi = groups + __popc(heads & ((1u << lane) - 1u));
+    for (int k = 0; k < GR_T / 32; ++k) {
+      if (k < wid) gi += warp_sum[k];
+      groups += warp_sum[k];
+    }
+    if (head) {
+      first[gi] = i;
+      base[gi] = row;
+      atomicAdd(&cnt[row], 1);
+    }
+  }
+  block_exclusive_scan(cnt, nf, warp_sum);
+  if (tid == 0) {
+    cnt[nf] = groups;
+    first[groups] = K;
+    w.groups[blockIdx.x] = groups;
+  }
+  __syncthreads();
+  for (int i = tid; i <= nf; i += GR_T) ptr[i] = cnt[i];
+  for (int b = tid; b < nf / GR_ROWS; b += GR_T) {
+    const int f0 = b * GR_ROWS;
+    bool u = cnt[max(f0 - GR_W + 1, 0)] != cnt[f0 + GR_ROWS];
+    if (b == 0) u = u || cnt[nf - GR_W + 1] != cnt[nf];  // groups that wrap around
+    used[b] = u;
+  }
+}
+
+// E[group][column]: the direct x phases, summed over the group's atoms, and the groups' spreading
+// weights.  A CTA takes 128 columns of every gridDim.y-th chunk of 16 groups of one job.
+__global__ void __launch_bounds__(128) k_grid_phases(GridPlanDev gp, SpeciesSet spset, TxGrid g, int job0,
+                                                     int col0, GridWork w) {
+  const int h = col0 + blockIdx.x * 128 + threadIdx.x, job = job0 + blockIdx.z;
+  const int4 jb = gp.jobs[job];
+  const double* pos = spset.k[jb.x & 3].pos + 2L * jb.z;
+  const int* order = w.order + gp.atom_beg[job];
+  const int* first = w.first + gp.atom_beg[job] + job;
+  float* wgt = reinterpret_cast<float*>(w.wgt + 2L * gp.atom_beg[job]);
+  float2* ex = w.ex + (long)blockIdx.z * w.kmax * w.ex_cols + (h - col0);
+  const int groups = w.groups[job];
+  // half: column h holds kx = h dkx, the last of them +p_w / 2 (the grid's own -p_w / 2 is its
+  // conjugate); columns beyond ``cols`` pad the pitch
+  const double kx = h >= w.cols ? 0.0
+                    : !w.half   ? g.kx_axis[h]
+                    : 2 * h < g.p_w ? g.kx_axis[g.p_w / 2 + h]
+                                    : -g.kx_axis[0];
+  for (int q0 = blockIdx.y * 16; q0 < groups; q0 += gridDim.y * 16) {
+    if (h < 128) {  // thread (q, k): weight k of group q
+      const int q = q0 + threadIdx.x / GR_W, k = threadIdx.x % GR_W;
+      if (q < groups) {
+        const double v = fine_row(pos[2L * order[first[q]] + 1], gp.dky, 2 * g.p_h);
+        const double d = (ceil(v - GR_W / 2) + k - v) / (GR_W / 2);
+        wgt[GR_W * q + k] = (float)(bessel_i0(GR_BETA * sqrt(fmax(1.0 - d * d, 0.0))) * (1.0 / bessel_i0(GR_BETA)));
+      }
+    }
+    if (h >= w.pitch) continue;
+    for (int q = q0; q < min(q0 + 16, groups); ++q) {
+      float2 s = make_float2(0.f, 0.f);
+      for (int i = first[q]; i < first[q + 1]; ++i) {
+        const double* p = pos + 2L * order[i];
+        s = cadd(s, phase_of(kx * p[0] + (w.half ? 0.0 : gp.sy * p[1])));
+      }
+      ex[(long)q * w.ex_cols] = s;
     }
   }
 }
 
-// Row pass: forward FFTs of the fine-grid rows of parity ex = 0 and 1 of one (job, ey, qy)
-// (p_w = N points of fixed-point pairs, 16 bytes each) in one CTA, then
-//   out[c] = ax[c][0] FFT(row_0)[k] + ax[c][1] FFT(row_1)[k],  k = (c + N/2) mod N,
-// written as complex64 over the first half of the ex = 0 row.  Transform g of a CTA takes parity
-// g & 1; the partner's spectrum comes through shared memory.  A fine row that no atom touched
-// (row_used == 0; most rows of a crystal, whose atoms sit on lattice rows) is zero and so is its
-// transform: the pair skips all work (from N = 256, where a pair never shares a warp with
-// another pair's warp-level barriers).  A pair that ran zeroes the second half of both its rows;
-// the first halves of all rows (where the column pass writes) and the flags are cleared in bulk
-// before each batch.  (A 128-register bound: the forward transform of a 16-byte-per-point row
-// does not fit 96.)
-template <int N>
-struct GridRowCfg {
-  static constexpr int P = RowCfg<N>::P, T = RowCfg<N>::T;
-  static constexpr int G = RowCfg<N>::G < 2 ? 2 : RowCfg<N>::G;
-  static constexpr int MINB = (512 / (G * T) > 0) ? 512 / (G * T) : 1;
-};
-template <int N>
-__global__ void __launch_bounds__(GridRowCfg<N>::G * GridRowCfg<N>::T, GridRowCfg<N>::MINB)
-    k_grid_rows(void* __restrict__ grid, const unsigned* __restrict__ row_used, const float4* __restrict__ ax, int p_h,
-                const float2* __restrict__ tw) {
-  constexpr int P = GridRowCfg<N>::P, T = GridRowCfg<N>::T, G = GridRowCfg<N>::G;
-  extern __shared__ float2 sh[];
-  float2* s_tw = sh;
-  float2* s_x = sh + Fft<N>::tw_size;
-  const int g = threadIdx.x / T, j = threadIdx.x - g * T, ex = g & 1;
-  const long pair = (long)blockIdx.x * (G / 2) + (g >> 1);
-  const long qy = pair % p_h, t = pair / p_h;                 // t = 2 job + ey
-  const long row0 = ((t >> 1) * 4 + 2 * (t & 1)) * p_h + qy;  // plane (ey, 0), row qy
-  // fine row 2 qy + ey of job t / 2
-  const bool live = N < 256 || row_used[(t >> 1) * 2 * p_h + 2 * qy + (t & 1)] != 0u;
-  longlong2* src = static_cast<longlong2*>(grid) + (row0 + ex * p_h) * N;
-  float2 v[P];
-  if (live) {
+// Adds weight times x of a group whose first fine row lies D rows from the block's.
+template <int D>
+__device__ __forceinline__ void spread_at(float2 (&acc)[GR_ROWS], const float* wt, float2 x) {
 #pragma unroll
-    for (int m = 0; m < P; ++m) {
-      const longlong2 q = src[j + m * T];
-      v[m] = make_float2(__ll2float_rn(q.x) * GR_UNFIX, __ll2float_rn(q.y) * GR_UNFIX);
+  for (int k = 0; k < GR_W; ++k)
+    if (D + k >= 0 && D + k < GR_ROWS) acc[D + k] = __ffma2_rn(make_float2(wt[k], wt[k]), x, acc[D + k]);
+}
+
+// One block of GR_ROWS fine rows of one job and 128 columns, a column per thread: the groups that
+// reach the block in sorted order.  All lanes take the same group, so its offset picks one of the 23
+// unrolled bodies without divergence and the weights are uniform loads; E is loaded four groups
+// ahead of its use.
+__global__ void __launch_bounds__(128) k_grid_spread(GridPlanDev gp, int p_h, int job0, int col0, GridWork w) {
+  const int nf = 2 * p_h, f0 = blockIdx.y * GR_ROWS, job = job0 + blockIdx.z;
+  const int h = col0 + blockIdx.x * 128 + threadIdx.x;
+  if (!w.used[(long)job * (nf / GR_ROWS) + blockIdx.y]) return;
+  const int hc = min(h, w.pitch - 1);
+  const int* __restrict__ ptr = w.ptr + (long)job * (nf + 1);
+  const int* __restrict__ base = w.base + gp.atom_beg[job];
+  const float4* __restrict__ wgt = w.wgt + 2L * gp.atom_beg[job];
+  const float2* __restrict__ ex = w.ex + (long)blockIdx.z * w.kmax * w.ex_cols + (hc - col0);
+  float2 acc[GR_ROWS];
+#pragma unroll
+  for (int t = 0; t < GR_ROWS; ++t) acc[t] = make_float2(0.f, 0.f);
+  for (int wrap = f0 == 0 ? 1 : 0; wrap >= 0; --wrap) {
+    const int lo = ptr[wrap ? nf - GR_W + 1 : max(f0 - GR_W + 1, 0)], hi = ptr[wrap ? nf : f0 + GR_ROWS];
+    const int shift = (wrap ? nf : 0) + f0;
+    for (int q0 = lo; q0 < hi; q0 += 4) {
+      float2 x[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = q0 + i < hi ? __ldg(ex + (long)(q0 + i) * w.ex_cols) : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (q0 + i >= hi) break;
+        const float4 wa = __ldg(wgt + 2 * (q0 + i)), wb = __ldg(wgt + 2 * (q0 + i) + 1);
+        const float wt[GR_W] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+        switch (__ldg(base + q0 + i) - shift) {
+#define TOTEM_SPREAD(D) \
+  case D: spread_at<D>(acc, wt, x[i]); break;
+          TOTEM_SPREAD(-7) TOTEM_SPREAD(-6) TOTEM_SPREAD(-5) TOTEM_SPREAD(-4) TOTEM_SPREAD(-3) TOTEM_SPREAD(-2)
+          TOTEM_SPREAD(-1) TOTEM_SPREAD(0) TOTEM_SPREAD(1) TOTEM_SPREAD(2) TOTEM_SPREAD(3) TOTEM_SPREAD(4)
+          TOTEM_SPREAD(5) TOTEM_SPREAD(6) TOTEM_SPREAD(7) TOTEM_SPREAD(8) TOTEM_SPREAD(9) TOTEM_SPREAD(10)
+          TOTEM_SPREAD(11) TOTEM_SPREAD(12) TOTEM_SPREAD(13) TOTEM_SPREAD(14) TOTEM_SPREAD(15)
+#undef TOTEM_SPREAD
+        }
+      }
     }
   }
-  load_twiddles<N>(s_tw, tw);
-  __syncthreads();  // every point of the CTA's rows is in registers before any is overwritten
-  const RowLayout<N> L;
-  if (live) {
-    // clear what the next batch's bulk clear leaves out: the second half of both rows
+  if (h >= w.pitch) return;
+  float2* dst = w.fine + ((long)blockIdx.z * nf + f0) * w.pitch + h;
 #pragma unroll
-    for (int m = P / 2; m < P; ++m) src[j + m * T] = make_longlong2(0, 0);
-    fft_regs<N, false>(v, j, g, s_tw, s_x, RowLayout<N>(), group_sync<N>(g));
-#pragma unroll
-    for (int m = 0; m < P; ++m) s_x[L(g, j + m * T)] = v[m];
-  }
-  __syncthreads();
-  if (!live) return;  // the output row is still the zero the grid was cleared to
-  float2* dst = static_cast<float2*>(grid) + row0 * 2 * N;
-#pragma unroll
-  for (int m = 0; m < P; ++m) {
-    if ((m < P / 2) != (ex == 0)) continue;  // parity 0 finishes k < N/2, parity 1 the rest
-    const int k = j + m * T;
-    const float2 other = s_x[L(g ^ 1, k)];
-    const float2 x0 = ex ? other : v[m], x1 = ex ? v[m] : other;
-    const int c = (k + N / 2) & (N - 1);
-    const float4 a = ax[c];
-    dst[c] = cadd(cmul(make_float2(a.x, a.y), x0), cmul(make_float2(a.z, a.w), x1));
-  }
+  for (int t = 0; t < GR_ROWS; ++t) dst[(long)t * w.pitch] = acc[t];
 }
 
-// Forward FFT of the columns of pitched planes (width columns, rows ``pitch`` apart).  Plane pl is
-// (job pl / 2, parity ey = pl % 2); its row q is fine row 2 q + ey, which is zero when no atom
-// touched it (row_used == 0: the row pass left the cleared zeros there), so it is not read.
-template <int N>
-__global__ void __launch_bounds__(GridColCfg<N>::G * GridColCfg<N>::T, GridColCfg<N>::MINB)
-    k_grid_cols(float2* __restrict__ data, int width, long pitch, long plane_stride, const unsigned* __restrict__ row_used,
-                const float2* __restrict__ tw) {
-  constexpr int P = GridColCfg<N>::P, T = GridColCfg<N>::T, G = GridColCfg<N>::G;
-  extern __shared__ float2 sh[];
-  float2* s_tw = sh;
-  float2* s_x = sh + Fft<N>::tw_size;
-  const int j = threadIdx.x / G, g = threadIdx.x - j * G;
-  const int nblk = width / G;
-  const long pl = blockIdx.x / nblk;
-  const int cb = blockIdx.x - (int)pl * nblk;
-  float2* p = data + pl * plane_stride + cb * G + g;
-  const unsigned* used = row_used + (pl >> 1) * 2 * N + (pl & 1);  // row q: used[2 q]
-  load_twiddles<N>(s_tw, tw);
-  float2 v[P];
-#pragma unroll
-  for (int m = 0; m < P; ++m) {
-    const int q = j + m * T;
-    v[m] = __ldg(used + 2 * q) ? p[(long)q * pitch] : make_float2(0.f, 0.f);
-  }
-  __syncthreads();
-  fft_regs<N, false>(v, j, g, s_tw, s_x, ColLayout<N, G>(), SyncBlock());
-#pragma unroll
-  for (int m = 0; m < P; ++m) p[(long)(j + m * T) * pitch] = v[m];
-}
-
-// V(r, c) of slices s_lo.. from the transformed planes of jobs [j_lo, j_hi): per job the y
-// half-bin combination and deconvolution give S, then f_species(s^2) S is summed; PARAMETER *
-// APERTURE as in k_tx_species.  A slice whose first jobs ran in an earlier batch adds to what
-// that batch wrote.
-__global__ void __launch_bounds__(256) k_grid_combine(TxGrid g, SpeciesSet spset, GridPlanDev gp,
-                                                      const float2* __restrict__ grid, int s_lo, int j_lo, int j_hi,
-                                                      float2* __restrict__ out) {
+// V(r, c) of slices s_lo.. from the jobs [j_lo, j_hi): f_species(s^2) S summed over the jobs,
+// PARAMETER * APERTURE as in k_tx_species.  A slice whose first jobs ran in an earlier batch adds
+// to what that batch wrote.
+__global__ void __launch_bounds__(256) k_grid_combine(TxGrid g, SpeciesSet spset, GridPlanDev gp, GridWork w, int s_lo,
+                                                      int j_lo, int j_hi, float2* __restrict__ out) {
   const long plane = (long)g.p_h * g.p_w;
-  const long pitch = 2L * g.p_w, pstride = (long)g.p_h * pitch;
   const int s = s_lo + blockIdx.y;
   const int jb0 = max(gp.job_beg[s], j_lo), jb1 = min(gp.job_beg[s + 1], j_hi);
   const bool add = gp.job_beg[s] < j_lo;
   float2* dst = out + (long)s * plane;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < plane; i += (long)gridDim.x * blockDim.x) {
     const int r = (int)(i / g.p_w), c = (int)(i - (long)r * g.p_w);
-    const int qr = (r + g.p_h / 2) & (g.p_h - 1);
-    const float2 y0 = gp.ay[2 * r], y1 = gp.ay[2 * r + 1];
     const float s2 = g.s2[i];
     float2 acc = make_float2(0.f, 0.f);
     for (int jj = jb0; jj < jb1; ++jj) {
       const int4 jb = gp.jobs[jj];
-      const float2* F = grid + (long)(jj - j_lo) * 4 * pstride + (long)qr * pitch + c;
-      const float2 S = cadd(cmul(y0, F[0]), cmul(y1, F[2 * pstride]));
+      const ColumnOfS col(w, w.s + (long)(jj - j_lo) * (g.p_h + 1) * w.pitch, g.p_h, g.p_w, c);
+      float2 S = col.at(r);
+      S.y *= col.sign;
       float fr, fi;
       species_form(jb.x & 3, g, spset.k[jb.x & 3], jb.y, s2, i, fr, fi);
       acc.x = fmaf(fr, S.x, fmaf(-fi, S.y, acc.x));
@@ -503,28 +510,49 @@ __global__ void __launch_bounds__(256) k_grid_combine(TxGrid g, SpeciesSet spset
   }
 }
 
-template <int N>
-Status grid_rows(void* grid, const unsigned* row_used, long pairs, const float2* ax, int p_h, const float2* tw,
-                 cudaStream_t st) {
-  constexpr int T = GridRowCfg<N>::T, G = GridRowCfg<N>::G;
-  const size_t smem = sizeof(float2) * (Fft<N>::tw_size + RowLayout<N>::size(G));
-  TOTEM_TRY(ensure_smem((const void*)k_grid_rows<N>, smem));
-  if (pairs % (G / 2)) return Status::Err(TOTEM_ERR_UNSUPPORTED, "row count not a multiple of the row tile");
-  k_grid_rows<N><<<(unsigned)(pairs / (G / 2)), G * T, smem, st>>>(grid, row_used, reinterpret_cast<const float4*>(ax),
-                                                                   p_h, tw);
-  return cuda_status(cudaGetLastError(), "k_grid_rows");
+// Where the parts of the work memory lie (base may be null: sizes only); returns its bytes.
+// ``batch`` jobs in a batch.
+size_t grid_work(int p_h, int p_w, int half, int kmax, int jobs, long long atoms, int batch, char* base, GridWork* w) {
+  w->kmax = kmax;
+  w->half = half;
+  w->cols = half ? p_w / 2 + 1 : p_w;
+  w->pitch = (w->cols + 15) / 16 * 16;
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    char* p = base + off;
+    off += (bytes + 255) & ~size_t(255);
+    return p;
+  };
+  const size_t nj = jobs, na = (size_t)atoms, nb = batch, row = w->pitch * sizeof(float2);
+  w->wgt = reinterpret_cast<float4*>(take(na * 2 * sizeof(float4)));
+  w->bin = reinterpret_cast<int*>(take(na * sizeof(int)));
+  w->base = reinterpret_cast<int*>(take(na * sizeof(int)));
+  w->order = reinterpret_cast<int*>(take(na * sizeof(int)));
+  w->first = reinterpret_cast<int*>(take((na + nj) * sizeof(int)));
+  w->ptr = reinterpret_cast<int*>(take(nj * (2 * (size_t)p_h + 1) * sizeof(int)));
+  w->groups = reinterpret_cast<int*>(take(nj * sizeof(int)));
+  w->used = reinterpret_cast<unsigned char*>(take(nj * (2 * (size_t)p_h / GR_ROWS)));
+  // E is at most as large as two fine columns' worth of rows; jobs of more atoms take it in pieces
+  const long room = 4L * p_h * w->pitch / kmax / 128 * 128;
+  w->ex_cols = room >= w->pitch ? w->pitch : (int)std::max(room, 128L);
+  w->ex = reinterpret_cast<float2*>(take(nb * kmax * w->ex_cols * sizeof(float2)));
+  w->fine = reinterpret_cast<float2*>(take(nb * 2 * p_h * row));
+  w->s = reinterpret_cast<float2*>(take(nb * (p_h + 1) * row));
+  return off;
 }
 
-template <int N>
-Status grid_cols(float2* data, long planes, int width, long pitch, long plane_stride, const unsigned* row_used,
-                 const float2* tw, cudaStream_t st) {
-  constexpr int T = GridColCfg<N>::T, G = GridColCfg<N>::G;
-  const size_t smem = sizeof(float2) * (Fft<N>::tw_size + ColLayout<N, G>::size(G));
-  TOTEM_TRY(ensure_smem((const void*)k_grid_cols<N>, smem));
-  if (width % G) return Status::Err(TOTEM_ERR_UNSUPPORTED, "grid width not a multiple of the column tile");
-  k_grid_cols<N><<<(unsigned)(planes * (width / G)), G * T, smem, st>>>(data, width, pitch, plane_stride, row_used,
-                                                                          tw);
-  return cuda_status(cudaGetLastError(), "k_grid_cols");
+// Batches of whole slices of at most jobs_per_batch jobs; empty if a slice has more.
+std::vector<GridBatch> whole_slice_batches(const std::vector<int>& job_beg, int jobs_per_batch) {
+  std::vector<GridBatch> out;
+  const int slices = (int)job_beg.size() - 1;
+  for (int s = 0; s < slices;) {
+    int e = s + 1;
+    if (job_beg[e] - job_beg[s] > jobs_per_batch) return {};
+    while (e < slices && job_beg[e + 1] - job_beg[s] <= jobs_per_batch) ++e;
+    out.push_back(GridBatch{s, e, job_beg[s], job_beg[e]});
+    s = e;
+  }
+  return out;
 }
 
 __global__ void k_sign_exp(float2* __restrict__ data, long total, int p_h, int p_w, float sig) {
@@ -534,20 +562,15 @@ __global__ void k_sign_exp(float2* __restrict__ data, long total, int p_h, int p
     const int r = (int)(k / p_w), c = (int)(k % p_w);
     // ifftshift of the input == multiplication of the output by (-1)^(r+c) (even sizes only;
     // the uploader rejects odd grids, as the reference's quadrant-swap ifftShift assumes).
-    const float sgn = ((r + c) & 1) ? -1.f : 1.f;
-    float2 v = data[i];
-    const float re = sgn * v.x * sig, im = sgn * v.y * sig;
-    const float amp = expf(-im);
-    float sn, cs;
-    sincosf(re, &sn, &cs);
-    data[i] = make_float2(amp * cs, amp * sn);
+    data[i] = exp_i_sigma(data[i], r + c, sig);
   }
 }
 
 }  // namespace
 
-bool gridding_size_ok(int n) { return n >= 64 && n <= 4096 && (n & (n - 1)) == 0; }
-bool fused_fft_size_ok(int n) { return gridding_size_ok(n) || radix_window_ops(n) != nullptr; }
+bool fused_fft_size_ok(int n) {
+  return (n >= 64 && n <= 4096 && (n & (n - 1)) == 0) || radix_window_ops(n) != nullptr;
+}
 
 namespace {
 template <int N>
@@ -590,18 +613,24 @@ Status launch_tx_species(const TxGrid& g, const SpeciesSet& sp, float2* out, cud
 }
 
 std::vector<float2> grid_deconvolution(int n) {
-  // tau = pi M_sp / (n^2 R (R - 1/2)); the fine grid's FFT carries 1 / (R n) per axis
-  const double pi = 3.14159265358979323846;
-  const double tau = pi * GR_MSP / ((double)n * n * 2.0 * 1.5);
-  const double pre = std::sqrt(pi / tau) / (2.0 * n);
+  // transform of the spreading kernel at xi = k / (2 n): W sinh(z) / (z I0(beta))
+  const double pi = 3.14159265358979323846, i0 = bessel_i0(GR_BETA);
   std::vector<float2> t(2 * (size_t)n);
-  for (int c = 0; c < n; ++c) {
-    const double k = c - n / 2;
-    const double d = pre * std::exp(k * k * tau);
-    t[2 * c] = make_float2((float)d, 0.f);
-    t[2 * c + 1] = make_float2((float)(d * std::cos(pi * k / n)), (float)(-d * std::sin(pi * k / n)));
+  for (int r = 0; r < n; ++r) {
+    const double k = r - n / 2, a = pi * GR_W * k / (2.0 * n);
+    const double z = std::sqrt(GR_BETA * GR_BETA - a * a);
+    const double d = z * i0 / (GR_W * std::sinh(z));
+    t[2 * r] = make_float2((float)d, 0.f);
+    t[2 * r + 1] = make_float2((float)(d * std::cos(pi * k / n)), (float)(-d * std::sin(pi * k / n)));
   }
   return t;
+}
+
+GridBytes grid_bytes(int p_h, int p_w, int half, int kmax, int jobs, long long atoms) {
+  GridWork w;
+  const size_t tables = grid_work(p_h, p_w, half, kmax, jobs, atoms, 0, nullptr, &w);
+  // (each part of a batch is rounded up to 256 bytes as a whole, so the batch never needs more)
+  return GridBytes{tables, grid_work(p_h, p_w, half, kmax, jobs, atoms, 1, nullptr, &w) - tables};
 }
 
 std::vector<GridBatch> grid_batches(const std::vector<int>& job_beg, int jobs_per_batch) {
@@ -624,68 +653,85 @@ std::vector<GridBatch> grid_batches(const std::vector<int>& job_beg, int jobs_pe
   return out;
 }
 
+namespace {
+// One instantiation per transform length: F(n) returns the Status of the launch.
+#define TOTEM_GRID_DISPATCH(NN, FN, OP, ...)                                             \
+  [&]() -> Status {                                                                      \
+    switch (NN) {                                                                        \
+      case 64: return FN<64>(__VA_ARGS__);                                               \
+      case 128: return FN<128>(__VA_ARGS__);                                             \
+      case 256: return FN<256>(__VA_ARGS__);                                             \
+      case 512: return FN<512>(__VA_ARGS__);                                             \
+      case 1024: return FN<1024>(__VA_ARGS__);                                           \
+      case 2048: return FN<2048>(__VA_ARGS__);                                           \
+      case 4096: return FN<4096>(__VA_ARGS__);                                           \
+    }                                                                                    \
+    if (const WindowOps* o = radix_window_ops(NN)) return o->OP(__VA_ARGS__);            \
+    return Status::Err(TOTEM_ERR_UNSUPPORTED, "gridding builder: unsupported grid edge"); \
+  }()
+}  // namespace
+
 Status launch_tx_gridding(const TxGrid& g, const SpeciesSet& sp, const GridPlanDev& gp,
-                          const std::vector<int>& job_beg, const std::vector<int4>& jobs, const float2* tw_w,
-                          const float2* tw_h, void* scratch, size_t scratch_bytes, bool scratch_zero, float2* out,
-                          cudaStream_t st, int* launches) {
+                          const std::vector<int>& job_beg, int kmax, long long atoms, const float2* tw_w,
+                          const float2* tw_h, void* scratch, size_t scratch_bytes, bool finish, float sig, float2* out,
+                          cudaStream_t st, int* launches, bool* finished) {
+  *finished = false;
   if (g.slices == 0) return Status::Ok();
-  if (!gridding_size_ok(g.p_h) || !gridding_size_ok(g.p_w))
-    return Status::Err(TOTEM_ERR_UNSUPPORTED, "gridding builder needs power-of-two grids 64..4096");
   if ((int)job_beg.size() != g.slices + 1) return Status::Err(TOTEM_ERR_STATE, "gridding job table size");
   const long plane = (long)g.p_h * g.p_w;
-  const size_t job_bytes = grid_job_bytes(g.p_h, g.p_w);
-  const int per_batch = (int)std::min<size_t>(scratch_bytes / job_bytes, 65535);  // grid.y of the spread
-  if (per_batch < 1) return Status::Err(TOTEM_ERR_STATE, "gridding scratch below one job");
-  const long pitch = 2L * g.p_w, pstride = (long)g.p_h * pitch;
-  const size_t plane_bytes = (size_t)plane * 64;  // four planes of 16-byte points per job
-  unsigned* used = reinterpret_cast<unsigned*>(static_cast<char*>(scratch) + plane_bytes * per_batch);
-  // Between batches the kernels leave the second half of every fine row zero; new scratch is
-  // cleared whole once, and the first halves (dense after the column pass) and the row flags are
-  // cleared in bulk before each batch (a strided memset; clearing the first halves in the combine
-  // after reading was measured 7x slower than the combine itself).
-  if (!scratch_zero) TOTEM_CUDA(cudaMemsetAsync(scratch, 0, job_bytes * per_batch, st));
-  for (const GridBatch& b : grid_batches(job_beg, per_batch)) {
+  const int jobs = job_beg.back();
+  const GridBytes need = grid_bytes(g.p_h, g.p_w, gp.half, kmax, jobs, atoms);
+  if (scratch_bytes < need.tables + need.per_job) return Status::Err(TOTEM_ERR_STATE, "gridding scratch below one job");
+  // at most 65535: the job is a grid dimension
+  const int per_batch = (int)std::min<size_t>((scratch_bytes - need.tables) / need.per_job, 65535);
+  GridWork w;
+  grid_work(g.p_h, g.p_w, gp.half, kmax, jobs, atoms, per_batch, static_cast<char*>(scratch), &w);
+  std::vector<GridBatch> batches;
+  if (finish) batches = whole_slice_batches(job_beg, per_batch);
+  if (batches.empty()) {
+    finish = false;
+    batches = grid_batches(job_beg, per_batch);
+  }
+  if (jobs > 0) {
+    const size_t smem = sizeof(int) * (2 * (size_t)g.p_h + 1);
+    TOTEM_TRY(ensure_smem((const void*)k_grid_sort, smem));
+    k_grid_sort<<<jobs, GR_T, smem, st>>>(gp, sp, g.p_h, w);
+    TOTEM_TRY(cuda_status(cudaGetLastError(), "k_grid_sort"));
+    ++*launches;
+  }
+  for (const GridBatch& b : batches) {
     const int nj = b.j_hi - b.j_lo;
     if (nj > 0) {
-      TOTEM_CUDA(cudaMemset2DAsync(scratch, 16 * (size_t)g.p_w, 0, 8 * (size_t)g.p_w, 4 * (size_t)g.p_h * nj, st));
-      TOTEM_CUDA(cudaMemsetAsync(used, 0, sizeof(unsigned) * 2 * g.p_h * nj, st));
-      int most = 0;
-      for (int j = b.j_lo; j < b.j_hi; ++j) most = std::max(most, jobs[j].w - jobs[j].z);
-      const unsigned bx = (unsigned)std::min<long>(((long)most * GR_W + 255) / 256 + 1, 4096);
-      k_grid_spread<<<dim3(bx, nj), 256, 0, st>>>(gp, g.p_h, g.p_w, sp, b.j_lo,
-                                                  static_cast<unsigned long long*>(scratch), used);
-      TOTEM_TRY(cuda_status(cudaGetLastError(), "k_grid_spread"));
-      const long pairs = (long)nj * 2 * g.p_h, planes = (long)nj * 2;  // (job, ey) after the row pass
-      float2* f = static_cast<float2*>(scratch);
-      switch (g.p_w) {
-        case 64: TOTEM_TRY(grid_rows<64>(scratch, used, pairs, gp.ax, g.p_h, tw_w, st)); break;
-        case 128: TOTEM_TRY(grid_rows<128>(scratch, used, pairs, gp.ax, g.p_h, tw_w, st)); break;
-        case 256: TOTEM_TRY(grid_rows<256>(scratch, used, pairs, gp.ax, g.p_h, tw_w, st)); break;
-        case 512: TOTEM_TRY(grid_rows<512>(scratch, used, pairs, gp.ax, g.p_h, tw_w, st)); break;
-        case 1024: TOTEM_TRY(grid_rows<1024>(scratch, used, pairs, gp.ax, g.p_h, tw_w, st)); break;
-        case 2048: TOTEM_TRY(grid_rows<2048>(scratch, used, pairs, gp.ax, g.p_h, tw_w, st)); break;
-        case 4096: TOTEM_TRY(grid_rows<4096>(scratch, used, pairs, gp.ax, g.p_h, tw_w, st)); break;
+      for (int col0 = 0; col0 < w.pitch; col0 += w.ex_cols) {
+        const unsigned cx = (std::min(w.ex_cols, w.pitch - col0) + 127) / 128;
+        k_grid_phases<<<dim3(cx, (unsigned)std::min((kmax + 15) / 16, 1024), nj), 128, 0, st>>>(gp, sp, g, b.j_lo,
+                                                                                               col0, w);
+        TOTEM_TRY(cuda_status(cudaGetLastError(), "k_grid_phases"));
+        k_grid_spread<<<dim3(cx, 2 * g.p_h / GR_ROWS, nj), 128, 0, st>>>(gp, g.p_h, b.j_lo, col0, w);
+        TOTEM_TRY(cuda_status(cudaGetLastError(), "k_grid_spread"));
+        *launches += 2;
       }
-      switch (g.p_h) {
-        case 64: TOTEM_TRY(grid_cols<64>(f, planes, g.p_w, pitch, 2 * pstride, used, tw_h, st)); break;
-        case 128: TOTEM_TRY(grid_cols<128>(f, planes, g.p_w, pitch, 2 * pstride, used, tw_h, st)); break;
-        case 256: TOTEM_TRY(grid_cols<256>(f, planes, g.p_w, pitch, 2 * pstride, used, tw_h, st)); break;
-        case 512: TOTEM_TRY(grid_cols<512>(f, planes, g.p_w, pitch, 2 * pstride, used, tw_h, st)); break;
-        case 1024: TOTEM_TRY(grid_cols<1024>(f, planes, g.p_w, pitch, 2 * pstride, used, tw_h, st)); break;
-        case 2048: TOTEM_TRY(grid_cols<2048>(f, planes, g.p_w, pitch, 2 * pstride, used, tw_h, st)); break;
-        case 4096: TOTEM_TRY(grid_cols<4096>(f, planes, g.p_w, pitch, 2 * pstride, used, tw_h, st)); break;
-      }
-      *launches += 3;
+      TOTEM_TRY(TOTEM_GRID_DISPATCH(g.p_h, grid_cols, grid_cols, w, b.j_lo, nj, gp.ay, tw_h, st));
+      ++*launches;
+    }
+    if (finish) {
+      float2* first = out + (long)b.s_lo * plane;
+      TOTEM_TRY(TOTEM_GRID_DISPATCH(g.p_h, grid_cols_inv, grid_cols_inv, g, sp, gp, w, b.s_lo, b.s_hi, b.j_lo, out,
+                                    tw_h, st));
+      TOTEM_TRY(TOTEM_GRID_DISPATCH(g.p_w, rows_exp, tx_rows_exp, first, (long)(b.s_hi - b.s_lo) * g.p_h, tw_w, sig,
+                                    st));
+      *launches += 2;
+      continue;
     }
     const unsigned cx = (unsigned)std::min<long>((plane + 255) / 256, 2048);
     for (int s0 = b.s_lo; s0 < b.s_hi; s0 += 65535) {
       const int ns = std::min(b.s_hi - s0, 65535);
-      k_grid_combine<<<dim3(cx, ns), 256, 0, st>>>(g, sp, gp, static_cast<const float2*>(scratch), s0, b.j_lo,
-                                                   b.j_hi, out);
+      k_grid_combine<<<dim3(cx, ns), 256, 0, st>>>(g, sp, gp, w, s0, b.j_lo, b.j_hi, out);
       TOTEM_TRY(cuda_status(cudaGetLastError(), "k_grid_combine"));
       ++*launches;
     }
   }
+  *finished = finish;
   return Status::Ok();
 }
 

@@ -14,6 +14,17 @@ namespace {
 template <int N>
 using GridColCfg = ColCfg<N, 4, (N == 4096) ? 4 : 0>;
 
+// exp(i sig V) of the transformed pixel v whose row and column index add up to an even or odd rc:
+// (-1)^rc carries the ifftshift of the input (even sizes).
+__device__ __forceinline__ float2 exp_i_sigma(float2 v, int rc, float sig) {
+  const float sgn = (rc & 1) ? -1.f : 1.f;
+  const float re = sgn * v.x * sig, im = sgn * v.y * sig;
+  const float amp = expf(-im);
+  float sn, cs;
+  sincosf(re, &sn, &cs);
+  return make_float2(amp * cs, amp * sn);
+}
+
 // In-place inverse FFT of rows of length N (RowCfg<N>::G rows per CTA).
 template <int N>
 __global__ void __launch_bounds__(RowCfg<N>::G * RowCfg<N>::T, RowCfg<N>::MINB) k_fft_rows_inv(float2* __restrict__ data,
@@ -57,12 +68,7 @@ __global__ void __launch_bounds__(GridColCfg<N>::G * GridColCfg<N>::T, GridColCf
 #pragma unroll
   for (int m = 0; m < P; ++m) {
     const int r = j + m * T;
-    const float sgn = ((r + c) & 1) ? -1.f : 1.f;
-    const float re = sgn * v[m].x * sig, im = sgn * v[m].y * sig;
-    const float amp = expf(-im);
-    float sn, cs;
-    sincosf(re, &sn, &cs);
-    p[(long)r * p_w] = make_float2(amp * cs, amp * sn);
+    p[(long)r * p_w] = exp_i_sigma(v[m], r + c, sig);
   }
 }
 

@@ -1,5 +1,5 @@
 """Transmission build time of the two builders for separable grids: the direct per-species sums
-(O(atoms x pixels)) and Gaussian gridding + FFT (O(atoms + pixels log pixels)), on SrTiO3 [001]
+(O(atoms x pixels)) and gridding + FFT (O(atoms x width + pixels log pixels)), on SrTiO3 [001]
 supercells that fill the potential grid (the serving workload's specimens), through a resident
 session.  Prints one JSON line per grid with both times, the speed-up and the relative L2
 difference of the two transmission stacks (on the first ``--check-slices`` slices).
