@@ -190,6 +190,10 @@ std::vector<float2> stage_twiddles(int n);
 // whatever the wave was.  The reference's propagator is cut at 2/3 of Nyquist
 // (ToTEM_submit_v1.m:1558-1564): band = N / 3.
 int spectral_band(const double* re, const double* im, int h, int w);
+// The same for rows: the largest index distance from DC of a row holding a non-zero entry, and
+// whether an n x n window's passes may take its rows BandRows<n> (fft.cuh) as zero.
+int spectral_row_band(const double* re, const double* im, int h, int w);
+bool band_rows_ok(int n, int row_band);
 // Column tiles [z0, z0 + nskip) left out of a column-pass launch.
 struct TileSkip {
   int z0 = 0, nskip = 0;
@@ -229,6 +233,7 @@ struct SliceLoopArgs {
   int col_variant = 0;             // column-pass variant (multislice.cu, col_pass)
   int t_bf16 = 0;                  // the transmission slices are bfloat16 pairs, not complex64
   int skip_band = 0;               // 1: the passes leave out band_columns(n) (band_skip_ok)
+  int skip_rows = 0;               // 1: the propagator is zero on the rows BandRows<n> (band_rows_ok)
   int row_variant = 0;             // row-pass variant (multislice.cu, row_pass)
 };
 // Number of column tiles per item (detector partial sums per probe) of a column-pass variant.
@@ -261,6 +266,7 @@ struct GroupDesc {
   int n;                        // window edge (the mixed-size kernels dispatch on it)
   int skip_band;                // 1: this group leaves out band_columns(n) in every pass
   TileSkip skip;                // its zero-band tiles (band_tiles), empty when skip_band is 0
+  int skip_rows;                // 1: its propagator is zero on the rows BandRows<n>
 };
 Status launch_row_groups(int n, const GroupDesc* groups, const int* item_begin, int ngroups, long items, int tick,
                          const float2* tw, cudaStream_t st);

@@ -444,6 +444,7 @@ Status totem_session::upload_args(const TotemStemArgs* a, bool stem) {
     TOTEM_TRY(upload(probe, pr, st));
     TOTEM_TRY(upload(prop, hp, st));
     band = (h == w) ? totem::spectral_band(a->prop_re, a->prop_im, h, w) : (1 << 30);
+    row_band = (h == w) ? totem::spectral_row_band(a->prop_re, a->prop_im, h, w) : (1 << 30);
     // exit detector: ifftshift(aper) (the reference shifts the wave instead, cuda_source_lobato.cu:1415)
     std::vector<float> me(vol * std::max(aper_num, 1)), mm;
     for (int q = 0; q < aper_num; ++q)
@@ -698,6 +699,8 @@ Status totem_session::slice_loop(int path, int batch, int col_variant, int t_sto
   const bool skip_band = fused && totem::band_skip_enabled() && t_storage == TOTEM_T_COMPLEX64 &&
                          totem::band_skip_ok(h, band, col_variant);
   const totem::TileSkip skip = skip_band ? totem::band_tiles(h, nblk) : totem::TileSkip();
+  const bool skip_rows = fused && totem::band_skip_enabled() && t_storage == TOTEM_T_COMPLEX64 &&
+                         totem::band_rows_ok(h, row_band);
   TOTEM_TRY(psi.ensure((size_t)B * vol * sizeof(float2)));
   TOTEM_TRY(part.ensure((size_t)n_events * B * aper_num * nblk * sizeof(double)));
   TOTEM_TRY(acc.ensure((size_t)n_events * w_num * ad * sizeof(double)));
@@ -729,6 +732,7 @@ Status totem_session::slice_loop(int path, int batch, int col_variant, int t_sto
         s.col_variant = col_variant;
         s.t_bf16 = (t_storage == TOTEM_T_BF16);
         s.skip_band = skip_band ? 1 : 0;
+        s.skip_rows = skip_rows ? 1 : 0;
         s.row_variant = row_variant;
         TOTEM_TRY(prof_begin());
         TOTEM_TRY(totem::launch_row_pass(s, tslice(0), true, stream));
@@ -797,7 +801,7 @@ Status totem_session::slice_loop(int path, int batch, int col_variant, int t_sto
     // what the launches embed: sizes, buffer addresses and the detection events
     std::vector<long long> key = {h, items_total, B, slices, col_variant, t_storage, n_events, exit_event, aper_num,
                                   w_num, depth, nblk, L, p_h, p_w, begin_row, begin_col, step, width_red,
-                                  (long long)tslice_bytes, skip_band ? 1 : 0, row_variant};
+                                  (long long)tslice_bytes, skip_band ? 1 : 0, skip_rows ? 1 : 0, row_variant};
     for (const void* q : {(const void*)psi.p, (const void*)part.p, (const void*)acc.p, (const void*)probe.p,
                           (const void*)prop.p, (const void*)tw_n.p, (const void*)mask_mid.p, (const void*)mask_exit.p,
                           Tslices, (const void*)gfsf_d.p, (const void*)out_result.p, (const void*)out_mid.p})
@@ -951,6 +955,10 @@ Status totem_session::hrtem(const TotemHrtemArgs* hr, TotemHrtemOut* out) {
                  totem::band_skip_ok(n, totem::spectral_band(hr->prop_re, hr->prop_im, n, n), 0))
                     ? 1
                     : 0;
+  s.skip_rows = (totem::band_skip_enabled() && hr->t_storage == TOTEM_T_COMPLEX64 &&
+                 totem::band_rows_ok(n, totem::spectral_row_band(hr->prop_re, hr->prop_im, n, n)))
+                    ? 1
+                    : 0;
   auto tslice = [&](int k) { return static_cast<const char*>(Tslices) + (size_t)k * tslice_bytes; };
   // psi = wave .* T_0, then per slice FFT2 .* psf_fft IFFT2 .* T_{k+1}; the last column pass keeps
   // the spectrum FFT2(psi_{S-1} .* T) .* psf_fft, whose IFFT2 is the exit wave
@@ -1079,6 +1087,7 @@ Status totem_session::cbed(double* pattern) {
     s.psi = ps; s.probe = probe.as<float2>(); s.prop = prop.as<float2>();
     s.tw = tw_n.as<float2>(); s.aper_num = 0;
     s.skip_band = (totem::band_skip_enabled() && totem::band_skip_ok(h, band, 0)) ? 1 : 0;
+    s.skip_rows = (totem::band_skip_enabled() && totem::band_rows_ok(h, row_band)) ? 1 : 0;
     TOTEM_TRY(totem::launch_row_pass(s, Tp, true, stream));
     for (int k = 0; k < slices; ++k) {
       TOTEM_TRY(totem::launch_col_pass(s, k == slices - 1 ? 4 | 8 : 0, stream));

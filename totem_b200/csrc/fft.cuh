@@ -26,18 +26,20 @@
 
 namespace totem {
 
-// Complex arithmetic on (re, im) pairs with sm_100's packed FP32 instructions (two IEEE FP32
-// operations per lane, round-to-nearest, the same results as the scalar forms).
+// Complex arithmetic on (re, im) pairs: sums with sm_100's packed FP32 instructions (two IEEE FP32
+// operations per lane), products as four scalar ones.  A packed product needs (a.x, a.x), (a.y, a.y)
+// and (-b.y, b.x) as register pairs, six moves the scalar form does without; it occupies the FMA
+// pipe as long, rounds the same, and made the slice loop 3.3 / 1.3 / 1.9 / 0.3 % faster at 256^2 /
+// 512^2 / 1024^2 / 2048^2.  (Sums as scalars too: 7 % slower at 256^2 and 8 % at 512^2.)
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
 __device__ __forceinline__ float2 cscale(float2 a, float s) { return __fmul2_rn(a, make_float2(s, s)); }
-// a * b = a.x * (b.x, b.y) + a.y * (-b.y, b.x)
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
-  return __ffma2_rn(make_float2(a.x, a.x), b, __fmul2_rn(make_float2(a.y, a.y), make_float2(-b.y, b.x)));
+  return make_float2(fmaf(a.x, b.x, -(a.y * b.y)), fmaf(a.x, b.y, a.y * b.x));
 }
-// a * conj(b) = a.x * (b.x, -b.y) + a.y * (b.y, b.x)
+// a * conj(b)
 __device__ __forceinline__ float2 cmulc(float2 a, float2 b) {
-  return __ffma2_rn(make_float2(a.x, a.x), make_float2(b.x, -b.y), __fmul2_rn(make_float2(a.y, a.y), make_float2(b.y, b.x)));
+  return make_float2(fmaf(a.x, b.x, a.y * b.y), fmaf(a.x, -b.y, a.y * b.x));
 }
 // a + s * (-i b) for s = +1 / -1 (forward) or a + s * (+i b) (inverse): the radix-4 cross term
 template <bool INV, int S>
@@ -88,7 +90,8 @@ constexpr double ce_cos_frac(int e, int R) {
 constexpr double ce_sin_frac(int e, int R) { return ce_cos_frac(4 * (e % R) - R, 4 * R); }
 
 // x * W_R^e (forward: exp(-2 pi i e/R)); inverse uses the conjugate.  Trivial angles are exact.
-template <int E, int R, bool INV>
+// EXACT_PRODUCT: odd eighths as a complex product instead of a scaled sum.
+template <int E, int R, bool INV, bool EXACT_PRODUCT = false>
 __device__ __forceinline__ float2 twiddle_const(float2 x) {
   constexpr int e = ((E % R) + R) % R;
   constexpr float r2 = 0.70710678118654752440f;
@@ -100,13 +103,13 @@ __device__ __forceinline__ float2 twiddle_const(float2 x) {
     return make_float2(-x.x, -x.y);
   } else if constexpr (4 * e == 3 * R) {  // +i (forward)
     return INV ? make_float2(x.y, -x.x) : make_float2(-x.y, x.x);
-  } else if constexpr (8 * e == R) {  // (1 -/+ i)/sqrt2 = (x + rot x) / sqrt2
+  } else if constexpr (!EXACT_PRODUCT && 8 * e == R) {  // (1 -/+ i)/sqrt2 = (x + rot x) / sqrt2
     return cscale(cadd_rot<INV, 1>(x, x), r2);
-  } else if constexpr (8 * e == 3 * R) {  // (-1 -/+ i)/sqrt2
+  } else if constexpr (!EXACT_PRODUCT && 8 * e == 3 * R) {  // (-1 -/+ i)/sqrt2
     return cscale(cadd_rot<INV, 1>(make_float2(-x.x, -x.y), x), r2);
-  } else if constexpr (8 * e == 5 * R) {  // (-1 +/- i)/sqrt2
+  } else if constexpr (!EXACT_PRODUCT && 8 * e == 5 * R) {  // (-1 +/- i)/sqrt2
     return cscale(cadd_rot<INV, -1>(make_float2(-x.x, -x.y), x), r2);
-  } else if constexpr (8 * e == 7 * R) {  // (1 +/- i)/sqrt2
+  } else if constexpr (!EXACT_PRODUCT && 8 * e == 7 * R) {  // (1 +/- i)/sqrt2
     return cscale(cadd_rot<INV, -1>(x, x), r2);
   } else {
     constexpr float c = (float)ce_cos_frac(e, R);
@@ -134,6 +137,29 @@ __device__ __forceinline__ void dft4(float2* y) {
   y[2] = csub(b0, b2);
   y[1] = cadd_rot<INV, 1>(b1, d);   // b1 + (-/+ i) d
   y[3] = cadd_rot<INV, -1>(b1, d);  // b1 - (-/+ i) d
+}
+
+// dft4 of inputs of which the ones in Z (a bit mask, known at compile time) are zero.
+template <bool INV, int Z>
+__device__ __forceinline__ void dft4_sparse(float2* y) {
+  if constexpr (Z == 4 || Z == 6 || Z == 2) {
+    const float2 a = y[0], c = y[3];
+    const float2 b0 = Z == 2 ? cadd(a, y[2]) : a, b1 = Z == 2 ? csub(a, y[2]) : a;
+    if constexpr (Z == 4) {
+      const float2 b2 = cadd(y[1], c), d = csub(y[1], c);
+      y[0] = cadd(b0, b2);
+      y[2] = csub(b0, b2);
+      y[1] = cadd_rot<INV, 1>(b1, d);
+      y[3] = cadd_rot<INV, -1>(b1, d);
+    } else {  // y[1] = 0: b2 = y[3], d = -y[3]
+      y[0] = cadd(b0, c);
+      y[2] = csub(b0, c);
+      y[1] = cadd_rot<INV, -1>(b1, c);
+      y[3] = cadd_rot<INV, 1>(b1, c);
+    }
+  } else {
+    dft4<INV>(y);
+  }
 }
 
 template <bool INV>
@@ -172,7 +198,8 @@ __device__ __forceinline__ void static_for(F&& f) {
 }
 
 // Cooley-Tukey split R = A * B: n = n1 + A n2, X[k2 + B k1] = sum_n1 W_A^{n1 k1} W_R^{n1 k2} DFT_B(x[n1 + A .])[k2]
-template <int A, int B, bool INV>
+// Inputs x[ZLO .. ZHI-1] are zero (used where the inner transforms are radix 4).
+template <int A, int B, bool INV, int ZLO = 0, int ZHI = 0>
 __device__ __forceinline__ void dft_split(float2* x) {
   float2 y[A][B];
   static_for<0, A>([&](auto n1c) {
@@ -180,7 +207,13 @@ __device__ __forceinline__ void dft_split(float2* x) {
     float2 z[B];
 #pragma unroll
     for (int n2 = 0; n2 < B; ++n2) z[n2] = x[n1 + A * n2];
-    dft_r<B, INV>(z);
+    if constexpr (B == 4 && ZHI > ZLO) {
+      constexpr auto zero = [](int n) { return n >= ZLO && n < ZHI; };
+      constexpr int Z = zero(n1) + 2 * zero(n1 + A) + 4 * zero(n1 + 2 * A) + 8 * zero(n1 + 3 * A);
+      dft4_sparse<INV, Z>(z);
+    } else {
+      dft_r<B, INV>(z);
+    }
     static_for<0, B>([&](auto k2c) {
       constexpr int k2 = decltype(k2c)::value;
       y[n1][k2] = twiddle_const<n1 * k2, A * B, INV>(z[k2]);
@@ -238,6 +271,14 @@ constexpr int ce_odd_factor(int r) {  // smallest odd prime factor (r not a powe
   for (int p = 3; p <= r; p += 2)
     if (r % p == 0) return p;
   return r;
+}
+
+// dft_r with inputs ZLO .. ZHI-1 zero; radices without a short form compute with the zeros.
+template <int R, bool INV, int ZLO, int ZHI>
+__device__ __forceinline__ void dft_r_sparse(float2* x) {
+  if constexpr (R == 16) dft_split<4, 4, INV, ZLO, ZHI>(x);
+  else if constexpr (R == 32) dft_split<8, 4, INV, ZLO, ZHI>(x);
+  else dft_r<R, INV>(x);
 }
 
 template <int R, bool INV>
@@ -399,7 +440,8 @@ struct SyncNamed {  // one named barrier per group of NT threads (NT a multiple 
 #endif
 constexpr bool kTwiddleDerive = TOTEM_TW_DERIVE != 0;
 
-template <int N, int S, bool INV, class Layout, class Sync, class Hook>
+// Inputs v[ZLO .. ZHI-1] of stage 0 are zero (ZLO = ZHI: none).
+template <int N, int S, bool INV, int ZLO, int ZHI, class Layout, class Sync, class Hook>
 struct StageLoop {
   __device__ __forceinline__ static void run(float2 (&v)[Fft<N>::P], int j, int g, const float2* __restrict__ tw,
                                              float2* sm, const Layout& L, const Sync& sync, Hook& hook) {
@@ -429,7 +471,10 @@ struct StageLoop {
         static_for<0, Q>([&](auto qc) {
           constexpr int q = decltype(qc)::value;
           const float2 x = INV ? cmulc(v[q * R + r], w) : cmul(v[q * R + r], w);
-          v[q * R + r] = twiddle_const<r * q * T, Ns * R, INV>(x);
+          // EXACT_PRODUCT: in a radix-2 butterfly whose other output is not needed the scaled sum of a
+          // 1/8 rotation would be contracted into the butterfly's add, and round otherwise than where
+          // both outputs are needed
+          v[q * R + r] = twiddle_const<r * q * T, Ns * R, INV, R == 2>(x);
         });
       });
 #pragma unroll
@@ -447,7 +492,8 @@ struct StageLoop {
             v[q * R + r] = INV ? cmulc(v[q * R + r], w) : cmul(v[q * R + r], w);
           }
         }
-        dft_r<R, INV>(&v[q * R]);
+        if constexpr (S == 0 && Q == 1) dft_r_sparse<R, INV, ZLO, ZHI>(v);
+        else dft_r<R, INV>(&v[q * R]);
       }
     }
     if constexpr (LAST) {
@@ -491,7 +537,7 @@ struct StageLoop {
         }
       sync();  // the region is free for the next exchange
       if constexpr (S + 2 == Fft<N>::stages) hook();  // last exchange done: the region is free
-      StageLoop<N, S + 1, INV, Layout, Sync, Hook>::run(v, j, g, tw, sm, L, sync, hook);
+      StageLoop<N, S + 1, INV, 0, 0, Layout, Sync, Hook>::run(v, j, g, tw, sm, L, sync, hook);
     }
   }
 };
@@ -503,11 +549,12 @@ struct NoHook {
 // Unnormalised transform of one length-N sequence held as v[m] = x[j + m*T].  Every thread of
 // the transform group must call it (it synchronises through ``sync``).  ``hook()`` runs once,
 // right after the last shared-memory exchange, when this transform's region is no longer read
-// by the transform (used to prefetch the next operand into it).
-template <int N, bool INV, class Layout, class Sync, class Hook = NoHook>
+// by the transform (used to prefetch the next operand into it).  v[ZLO .. ZHI-1] are zero on entry
+// (the zero band of a band-limited wave): the first radix leaves their sums out.
+template <int N, bool INV, int ZLO = 0, int ZHI = 0, class Layout, class Sync, class Hook = NoHook>
 __device__ __forceinline__ void fft_regs(float2 (&v)[Fft<N>::P], int j, int g, const float2* tw, float2* sm,
                                          const Layout& L, const Sync& sync, Hook&& hook = Hook()) {
-  StageLoop<N, 0, INV, Layout, Sync, std::remove_reference_t<Hook>>::run(v, j, g, tw, sm, L, sync, hook);
+  StageLoop<N, 0, INV, ZLO, ZHI, Layout, Sync, std::remove_reference_t<Hook>>::run(v, j, g, tw, sm, L, sync, hook);
 }
 
 // 8-byte asynchronous global -> shared copies (each thread later reads only what it copied).
@@ -589,6 +636,15 @@ struct BandCols {
   static constexpr int K = N / 3;
   static constexpr int lo = (K + 1 + L - 1) / L * L;
   static constexpr int hi = ((N - K) / L * L > lo) ? (N - K) / L * L : lo;
+};
+
+// Rows [lo, hi) of a column of such a window that a propagator zero beyond the same distance leaves
+// zero, rounded inward to whole groups of T column-pass elements (no tile width to respect here).
+template <int N>
+struct BandRows {
+  static constexpr int T = Fft<N>::T, K = N / 3;
+  static constexpr int lo = (K + 1 + T - 1) / T * T;
+  static constexpr int hi = ((N - K) / T * T > lo) ? (N - K) / T * T : lo;
 };
 
 // Transform groups of T threads: within a warp when T divides 32, whole warps with a named barrier

@@ -160,6 +160,23 @@ int spectral_band(const double* re, const double* im, int h, int w) {
   return band;
 }
 
+int spectral_row_band(const double* re, const double* im, int h, int w) {
+  int band = 0;
+  for (int r = 0; r < h; ++r) {
+    const int dist = r < h - r ? r : h - r;
+    if (dist <= band) continue;
+    for (int c = 0; c < w; ++c)
+      if (re[(size_t)r * w + c] != 0.0 || im[(size_t)r * w + c] != 0.0) {
+        band = dist;
+        break;
+      }
+  }
+  return band;
+}
+
+// BandRows<n> starts at or beyond n / 3 + 1 and ends at or before n - n / 3 for every n
+bool band_rows_ok(int n, int row_band) { return row_band <= n / 3; }
+
 Status launch_combine(const double* acc, const double* gfsf, int w_num, long ad, double* out, cudaStream_t st) {
   if (ad == 0) return Status::Ok();
   k_combine<<<(unsigned)((ad + 255) / 256), 256, 0, st>>>(acc, gfsf, w_num, ad, out);

@@ -75,7 +75,7 @@ Status row_pass(const SliceLoopArgs& a, const void* tslice, cudaStream_t st) {
 // prefetching the propagator into shared memory (4.6 ms against 4.3 ms per 4096 probes) and an
 // 80-register cap (5.8 ms) were slower.
 // The launch covers the tiles outside [skip.z0, skip.z0 + skip.nskip) only.
-template <int N, bool PREFETCH, int CTAS128, int GW>
+template <int N, bool PREFETCH, int CTAS128, int GW, bool ROWS>
 __global__ void __launch_bounds__(ColCfg<N, CTAS128, GW>::G * ColCfg<N, CTAS128, GW>::T, ColCfg<N, CTAS128, GW>::MINB)
     k_col_pass(SliceLoopArgs a, int flags, TileSkip skip) {
   constexpr int G = ColCfg<N, CTAS128, GW>::G;
@@ -84,18 +84,30 @@ __global__ void __launch_bounds__(ColCfg<N, CTAS128, GW>::G * ColCfg<N, CTAS128,
   const int item = blockIdx.x / active, t = blockIdx.x - item * active;
   const int cb = t < skip.z0 ? t : t + skip.nskip;
   const ColInputs in{a.prop, a.mask_mid, a.mask_exit, a.aper_num, a.part_mid, a.part_exit};
-  col_tile<N, PREFETCH, G>(a.psi + (long)item * N * N, in, item, cb, flags, a.tw);
+  col_tile<N, PREFETCH, G, ROWS>(a.psi + (long)item * N * N, in, item, cb, flags, a.tw);
 }
 
-template <int N, bool PREFETCH, int CTAS128, int GW>
-Status col_pass_v(const SliceLoopArgs& a, int flags, cudaStream_t st) {
+template <int N, bool PREFETCH, int CTAS128, int GW, bool ROWS>
+Status col_pass_launch(const SliceLoopArgs& a, int flags, TileSkip skip, cudaStream_t st) {
   constexpr int G = ColCfg<N, CTAS128, GW>::G, T = ColCfg<N>::T;
   const size_t smem = sizeof(float2) * (Fft<N>::tw_size + ColLayout<N, G>::size(G));
-  TOTEM_TRY(ensure_smem((const void*)k_col_pass<N, PREFETCH, CTAS128, GW>, smem));
-  const TileSkip skip = a.skip_band ? band_tiles(N, N / G) : TileSkip();
-  k_col_pass<N, PREFETCH, CTAS128, GW>
+  TOTEM_TRY(ensure_smem((const void*)k_col_pass<N, PREFETCH, CTAS128, GW, ROWS>, smem));
+  k_col_pass<N, PREFETCH, CTAS128, GW, ROWS>
       <<<(unsigned)((long)a.items * (N / G - skip.nskip)), G * T, smem, st>>>(a, flags, skip);
-  TOTEM_TRY(cuda_status(cudaGetLastError(), "k_col_pass"));
+  return cuda_status(cudaGetLastError(), "k_col_pass");
+}
+
+// the zero rows (a.skip_rows) chosen at launch; windows without a band of rows skip nothing
+template <int N, bool PREFETCH, int CTAS128, int GW>
+Status col_pass_v(const SliceLoopArgs& a, int flags, cudaStream_t st) {
+  constexpr int G = ColCfg<N, CTAS128, GW>::G;
+  const TileSkip skip = a.skip_band ? band_tiles(N, N / G) : TileSkip();
+  bool rows = false;
+  if constexpr (BandRows<N>::hi > BandRows<N>::lo) {
+    rows = a.skip_rows != 0;
+    if (rows) TOTEM_TRY((col_pass_launch<N, PREFETCH, CTAS128, GW, true>(a, flags, skip, st)));
+  }
+  if (!rows) TOTEM_TRY((col_pass_launch<N, PREFETCH, CTAS128, GW, false>(a, flags, skip, st)));
   if ((flags & 8) && skip.nskip) {
     // a kept spectrum is stored whole: on the skipped columns it is exactly zero (the propagator is)
     const size_t pitch = (size_t)N * sizeof(float2);

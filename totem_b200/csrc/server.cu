@@ -58,6 +58,7 @@ struct Request {
   long long items = 0, items_left = 0;
   int nblk = 0;
   int skip_band = 0;                // its groups leave out the propagator's zero band
+  int skip_rows = 0;                // its propagator is zero on the rows BandRows<n>
   size_t item_bytes = 0;
   long long probe_slices = 0;
   double est = 0;                   // estimated device seconds (preparation order)
@@ -252,6 +253,7 @@ Status totem_server::prepare(Request* r) {
   r->items_left = r->items;
   r->nblk = totem::col_blocks(s->h);
   r->skip_band = (totem::band_skip_enabled() && totem::band_skip_ok(s->h, s->band, 0)) ? 1 : 0;
+  r->skip_rows = (totem::band_skip_enabled() && totem::band_rows_ok(s->h, s->row_band)) ? 1 : 0;
   r->item_bytes = (size_t)s->h * s->w * sizeof(float2) + (size_t)r->de.n_events * s->aper_num * r->nblk * sizeof(double);
   r->probe_slices = (long long)s->w_num * s->depth * s->slices;
   TOTEM_CUDA(cudaEventCreateWithFlags(&r->ready, cudaEventDisableTiming));
@@ -398,6 +400,7 @@ Status totem_server::tick_once(Lane& lane, bool* progressed) {
     x.exit_event = r->de.exit_event;
     x.n = n;
     x.skip_band = r->skip_band;
+    x.skip_rows = r->skip_rows;
     x.skip = r->skip_band ? totem::band_tiles(n, totem::col_blocks(n)) : totem::TileSkip();
     return Status::Ok();
   };

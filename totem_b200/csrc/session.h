@@ -199,6 +199,7 @@ struct totem_session {
   long long h2d_bytes = 0, d2h_bytes = 0;
   // band of the uploaded propagator (totem::spectral_band; n / 2 and above: no zero band)
   int band = 1 << 30;
+  int row_band = 1 << 30;  // totem::spectral_row_band
   // which implementations the last run used (TotemTiming.slice_path / tx_fft_path / tx_builder)
   int ran_slice_path = -1, ran_tx_fft = -1, ran_tx_builder = -1;
   int used_row_variant = 0, used_col_variant = 0;

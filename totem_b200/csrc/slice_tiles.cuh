@@ -79,7 +79,7 @@ __device__ __forceinline__ void row_tile(float2* __restrict__ psi_item, const vo
     for (int m = 0; m < P; ++m) v[m] = (m >= mlo && m < mhi) ? make_float2(0.f, 0.f) : prow[j + m * T];
   }
   __syncthreads();  // twiddles staged
-  if (!FIRST) fft_regs<N, true>(v, j, g, s_tw, s_x, L, sync, prefetch_t);
+  if (!FIRST) fft_regs<N, true, SKIP ? mlo : 0, SKIP ? mhi : 0>(v, j, g, s_tw, s_x, L, sync, prefetch_t);
   cp_async_wait_all();
 #pragma unroll
   for (int m = 0; m < P; ++m) {
@@ -138,11 +138,15 @@ struct ColInputs {
 
 // One CTA's share of a column pass: columns cb*G .. cb*G+G-1 of one probe's wave.  ``item`` is
 // the item's index in the partial-sum arrays.  flags: 1 mid detectors, 2 exit detectors,
-// 4 final pass (no inverse transform), 8 (with 4) store the spectrum.
-template <int N, bool PREFETCH, int G>
+// 4 final pass (no inverse transform), 8 (with 4) store the spectrum.  ROWS: the propagator is zero on
+// the rows BandRows<N>::lo .. hi-1 of every column, so the spectrum is set to zero there without
+// reading it, and the forward transform's outputs and the inverse's sums of zeros are left out.
+template <int N, bool PREFETCH, int G, bool ROWS>
 __device__ __forceinline__ void col_tile(float2* __restrict__ psi_item, const ColInputs& in, int item, int cb, int flags,
                                          const float2* __restrict__ tw) {
   constexpr int P = ColCfg<N>::P, T = ColCfg<N>::T;
+  constexpr int zlo = ROWS ? BandRows<N>::lo / T : 0, zhi = ROWS ? BandRows<N>::hi / T : 0;
+  constexpr auto zero = [](int m) { return m >= zlo && m < zhi; };
   extern __shared__ float2 sh[];
   float2* s_tw = sh;
   float2* s_x = sh + Fft<N>::tw_size;
@@ -163,17 +167,19 @@ __device__ __forceinline__ void col_tile(float2* __restrict__ psi_item, const Co
   if constexpr (!PREFETCH) {
     fft_regs<N, false>(v, j, g, s_tw, s_x, L, sync);
 #pragma unroll
-    for (int m = 0; m < P; ++m) v[m] = cmul(v[m], __ldg(in.prop + (long)(j + m * T) * N + c));
+    for (int m = 0; m < P; ++m)
+      v[m] = zero(m) ? make_float2(0.f, 0.f) : cmul(v[m], __ldg(in.prop + (long)(j + m * T) * N + c));
   } else {
     auto prefetch_h = [&]() {
 #pragma unroll
-      for (int m = 0; m < P; ++m) cp_async8(&s_x[L.pos(g, j, m)], in.prop + (long)(j + m * T) * N + c);
+      for (int m = 0; m < P; ++m)
+        if (!zero(m)) cp_async8(&s_x[L.pos(g, j, m)], in.prop + (long)(j + m * T) * N + c);
       cp_async_commit();
     };
     fft_regs<N, false>(v, j, g, s_tw, s_x, L, sync, prefetch_h);
     cp_async_wait_all();
 #pragma unroll
-    for (int m = 0; m < P; ++m) v[m] = cmul(v[m], s_x[L.pos(g, j, m)]);
+    for (int m = 0; m < P; ++m) v[m] = zero(m) ? make_float2(0.f, 0.f) : cmul(v[m], s_x[L.pos(g, j, m)]);
     sync();  // all propagator values read before the inverse transform reuses the region
   }
   if (flags & 3) {
@@ -190,7 +196,7 @@ __device__ __forceinline__ void col_tile(float2* __restrict__ psi_item, const Co
     }
     return;
   }
-  fft_regs<N, true>(v, j, g, s_tw, s_x, L, sync);
+  fft_regs<N, true, zlo, zhi>(v, j, g, s_tw, s_x, L, sync);
 #pragma unroll
   for (int m = 0; m < P; ++m) base[(long)(j + m * T) * N] = v[m];
 }
@@ -260,7 +266,13 @@ __device__ __forceinline__ void col_group_tile(const GroupDesc& d, int item, int
     flags |= 2 | 4;
     in.part_exit = d.part + d.exit_event * estride;
   }
-  col_tile<N, false, G>(d.psi + (long)item * N * N, in, item, cb, flags, tw);
+  if constexpr (BandRows<N>::hi > BandRows<N>::lo) {
+    if (d.skip_rows) {
+      col_tile<N, false, G, true>(d.psi + (long)item * N * N, in, item, cb, flags, tw);
+      return;
+    }
+  }
+  col_tile<N, false, G, false>(d.psi + (long)item * N * N, in, item, cb, flags, tw);
 }
 
 }  // namespace
