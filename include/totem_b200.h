@@ -123,8 +123,10 @@ enum {
 /* Engine options of one run (defaults: all zero). */
 typedef struct TotemRunOptions {
   int path;                        /* TOTEM_PATH_*                                              */
-  int batch;                       /* probes in flight per batch, 0 = the tuned choice (else up to
-                                      4 GiB of waves for the fused path, 1 GiB for cuFFT)         */
+  int batch;                       /* probes in flight per batch, in one sequence of batches; 0 = the
+                                      engine's choice: for the fused path one batch, or two
+                                      sequences of smaller ones on two streams, of at most the
+                                      tuned size (else 4 GiB of waves); 1 GiB for cuFFT          */
   int skip_transmission;           /* 1 = reuse the transmission built by an earlier run        */
   int profile;                     /* 1 = CUDA events around every slice-loop pass launch       */
   int col_variant;                 /* fused column pass: 0 = the tuned choice for this window and

@@ -656,7 +656,52 @@ Status totem_session::transmission_for(int t_storage, const void** t, size_t* sl
   return Status::Ok();
 }
 
-Status totem_session::slice_loop(int path, int batch, int col_variant, int t_storage, int* launches,
+namespace {
+// How the items of a fused run are split: ``chains`` (1 or 2) sequences of batches on as many
+// streams.  Two chains of batches whose waves stay in L2 together run faster than one launch over
+// all items streaming 4 GiB through HBM: each pass finds its waves in L2, and the partial last wave
+// of CTAs of one chain's short launch is filled by the other's.  (One chain of L2-sized batches is
+// slower than either: 1.38-1.44 us.)  Measured per probe*slice, one batch against two chains:
+// 128^2 0.0901 / 0.0786, 256^2 0.323 / 0.303, 400^2 1.150 / 1.060, 512^2 1.312 / 1.247, 640^2 3.654 /
+// 3.662, 800^2 6.345 / 6.344, 1280^2 16.77 / 16.11, 2048^2 39.88 / 38.31 us.
+//  * Waves of both chains together: 50 MB up to 576^2, 32 MB above (512^2 at 32 / 44 / 56 / 68 MB:
+//    1.291 / 1.253 / 1.247 / 1.253; 640^2 3.662 / 3.716 / 3.904 / 4.071).  Windows of which L2 does
+//    not hold two (2048^2) still gain from the overlap; eight a batch was best.
+//  * 1024^2 and 1536^2 windows stream faster than they run from L2 (5.96 against 6.30 us, 22.89
+//    against 23.70): one batch, unless there are too few to amortise it (1024^2: 8 / 16 / 30 items in
+//    one batch 6.63 / 6.82 / 6.41).
+//  * Below 1.5 M points in all, one launch does not fill the GPU and two only add launches (256^2, 8
+//    items 1.109 / 1.142, 16 items 0.722 / 0.715; 512^2, 4 items 3.39 / 3.34, 8 items 2.47 / 2.31).
+// ``cap`` bounds the probes of a batch (0: 4 GiB of waves).
+struct SlicePlan {
+  int chains = 1, batch = 1;
+};
+SlicePlan plan_chains(int n, long items, long cap) {
+  const double wave = (double)n * n * sizeof(float2);
+  if (cap <= 0) cap = std::max<long>(1, (long)((4ull << 30) / (size_t)wave));
+  SlicePlan p;
+  long b = std::min(cap, items);
+  const bool streams = (n == 1024 || n == 1536) && items * wave >= 0.35e9;
+  if (items >= 2 && (double)items * n * n >= 1.5 * 1048576 && !streams) {
+    const double in_l2 = (n <= 576 ? 25e6 : 16e6) / (wave * 2 / 3);  // a third of the columns are left out
+    p.chains = 2;
+    b = std::min(std::min(cap, (items + 1) / 2), in_l2 < 0.8 ? 8 : std::max<long>(1, std::lround(in_l2)));
+  }
+  long nb = (items + b - 1) / b;           // spread the items evenly over the batches,
+  if (p.chains == 2) nb += nb & 1;         // and the batches over the chains
+  p.batch = (int)((items + nb - 1) / nb);
+  return p;
+}
+}  // namespace
+
+Status totem_session::second_stream() {
+  if (stream2 == nullptr) TOTEM_CUDA(cudaStreamCreateWithFlags(&stream2, cudaStreamNonBlocking));
+  for (cudaEvent_t* e : {&fork_ev, &join_ev})
+    if (*e == nullptr) TOTEM_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  return Status::Ok();
+}
+
+Status totem_session::slice_loop(int path, int batch, bool batch_fixed, int col_variant, int t_storage, int* launches,
                                  int* batch_used, int row_variant) {
   const long items_total = (long)w_num * depth;
   const long ad = (long)aper_num * depth;
@@ -679,19 +724,21 @@ Status totem_session::slice_loop(int path, int batch, int col_variant, int t_sto
                        "1152, 1280, 1536, 1600)");
   ran_slice_path = fused ? TOTEM_PATH_FUSED : TOTEM_PATH_PLAIN;
   const size_t vol = (size_t)h * w;
-  int B = batch;
-  if (B <= 0) {
-    // Large batches win on B200: keeping a batch L2-resident between passes (<= ~64 MB) was
-    // measured slower than streaming a large batch through HBM, because wave tails dominate the
-    // short launches (SrTiO3 512^2: 24 probes 948 ms, 4096 probes 879 ms per request).
-    const size_t target = fused ? (4ull << 30) : (1ull << 30);
-    B = (int)std::max<size_t>(1, target / (vol * sizeof(float2)));
+  SlicePlan plan_b;
+  if (fused && !batch_fixed && !profiling) {
+    plan_b = plan_chains(h, items_total, batch);
+  } else {
+    plan_b.batch = batch;
+    if (batch <= 0) {
+      const size_t target = fused ? (4ull << 30) : (1ull << 30);
+      plan_b.batch = (int)std::max<size_t>(1, target / (vol * sizeof(float2)));
+    }
+    plan_b.batch = (int)std::min<long>(plan_b.batch, items_total);
+    // spread the items evenly over the batches
+    const long nb = (items_total + plan_b.batch - 1) / plan_b.batch;
+    plan_b.batch = (int)((items_total + nb - 1) / nb);
   }
-  B = (int)std::min<long>(B, items_total);
-  {  // spread the items evenly over the batches
-    const long nb = (items_total + B - 1) / B;
-    B = (int)((items_total + nb - 1) / nb);
-  }
+  const int B = plan_b.batch, chains = plan_b.chains;
   *batch_used = B;
   const int nblk = fused ? totem::col_blocks(h, col_variant) : 64;
   // the zero band of the propagator: columns the fused passes leave out, tiles the detector sums
@@ -701,11 +748,11 @@ Status totem_session::slice_loop(int path, int batch, int col_variant, int t_sto
   const totem::TileSkip skip = skip_band ? totem::band_tiles(h, nblk) : totem::TileSkip();
   const bool skip_rows = fused && totem::band_skip_enabled() && t_storage == TOTEM_T_COMPLEX64 &&
                          totem::band_rows_ok(h, row_band);
-  TOTEM_TRY(psi.ensure((size_t)B * vol * sizeof(float2)));
-  TOTEM_TRY(part.ensure((size_t)n_events * B * aper_num * nblk * sizeof(double)));
+  if (chains > 1) TOTEM_TRY(second_stream());
+  const size_t part_stride = (size_t)B * aper_num * nblk;  // one event of one chain
+  TOTEM_TRY(psi.ensure((size_t)chains * B * vol * sizeof(float2)));
+  TOTEM_TRY(part.ensure(chains * n_events * part_stride * sizeof(double)));
   TOTEM_TRY(acc.ensure((size_t)n_events * w_num * ad * sizeof(double)));
-  double* part_e = part.as<double>();
-  const size_t part_stride = (size_t)B * aper_num * nblk;
   totem::ScanGeom geo{begin_row, begin_col, step, width_red, depth, p_w};
   const float2* Tp = T.as<float2>();
   const size_t plane = (size_t)p_h * p_w;
@@ -717,16 +764,16 @@ Status totem_session::slice_loop(int path, int batch, int col_variant, int t_sto
   }
   auto tslice = [&](int k) { return static_cast<const char*>(Tslices) + (size_t)k * tslice_bytes; };
 
-  // Everything below is stream work only (no allocation, no host synchronisation), so a repeated
-  // fused run can replay it as one CUDA graph (see run_graphed).
-  auto enqueue = [&]() -> Status {
-    TOTEM_CUDA(cudaMemsetAsync(acc.p, 0, (size_t)n_events * w_num * ad * sizeof(double), stream));
-    for (long item0 = 0; item0 < items_total; item0 += B) {
+  auto enqueue_batches = [&]() -> Status {
+    int turn = 0;
+    for (long item0 = 0; item0 < items_total; item0 += B, turn = (turn + 1) % chains) {
+      const cudaStream_t st = turn == 0 ? stream : stream2;
+      double* part_e = part.as<double>() + turn * n_events * part_stride;
       const int items = (int)std::min<long>(B, items_total - item0);
       if (fused) {
         totem::SliceLoopArgs s;
         s.n = h; s.items = items; s.item0 = (int)item0; s.geo = geo; s.p_h = p_h;
-        s.psi = psi.as<float2>(); s.probe = probe.as<float2>(); s.prop = prop.as<float2>();
+        s.psi = psi.as<float2>() + turn * (size_t)B * vol; s.probe = probe.as<float2>(); s.prop = prop.as<float2>();
         s.tw = tw_n.as<float2>(); s.aper_num = aper_num;
         s.mask_mid = mask_mid.as<float>(); s.mask_exit = mask_exit.as<float>();
         s.col_variant = col_variant;
@@ -735,7 +782,7 @@ Status totem_session::slice_loop(int path, int batch, int col_variant, int t_sto
         s.skip_rows = skip_rows ? 1 : 0;
         s.row_variant = row_variant;
         TOTEM_TRY(prof_begin());
-        TOTEM_TRY(totem::launch_row_pass(s, tslice(0), true, stream));
+        TOTEM_TRY(totem::launch_row_pass(s, tslice(0), true, st));
         TOTEM_TRY(prof_end(0));
         ++*launches;
         for (int k = 0; k < slices; ++k) {
@@ -750,12 +797,12 @@ Status totem_session::slice_loop(int path, int batch, int col_variant, int t_sto
             s.part_exit = part_e + exit_event * part_stride;
           }
           TOTEM_TRY(prof_begin());
-          TOTEM_TRY(totem::launch_col_pass(s, flags, stream));
+          TOTEM_TRY(totem::launch_col_pass(s, flags, st));
           TOTEM_TRY(prof_end(1));
           ++*launches;
           if (k < slices - 1) {
             TOTEM_TRY(prof_begin());
-            TOTEM_TRY(totem::launch_row_pass(s, tslice(k + 1), false, stream));
+            TOTEM_TRY(totem::launch_row_pass(s, tslice(k + 1), false, st));
             TOTEM_TRY(prof_end(0));
             ++*launches;
           }
@@ -788,18 +835,38 @@ Status totem_session::slice_loop(int path, int batch, int col_variant, int t_sto
       }
       for (int e = 0; e < n_events; ++e) {
         TOTEM_TRY(totem::launch_det_reduce(part_e + e * part_stride, nblk, aper_num, items, (int)item0, depth,
-                                           acc.as<double>() + (size_t)e * w_num * ad, stream, skip));
+                                           acc.as<double>() + (size_t)e * w_num * ad, st, skip));
         ++*launches;
       }
     }
+    return Status::Ok();
+  };
+
+  // Everything below is stream work only (no allocation, no host synchronisation), so a repeated
+  // fused run can replay it as one CUDA graph (see run_graphed).  With two chains the batches go to
+  // the session's stream and its second one in turn, each with its own waves and partial sums.
+  auto enqueue = [&]() -> Status {
+    TOTEM_CUDA(cudaMemsetAsync(acc.p, 0, (size_t)n_events * w_num * ad * sizeof(double), stream));
+    if (chains > 1) {
+      TOTEM_CUDA(cudaEventRecord(fork_ev, stream));
+      TOTEM_CUDA(cudaStreamWaitEvent(stream2, fork_ev, 0));
+    }
+    const Status st = enqueue_batches();
+    if (chains > 1) {  // joined whether or not every launch succeeded: nothing outlives the run
+      TOTEM_CUDA(cudaEventRecord(join_ev, stream2));
+      TOTEM_CUDA(cudaStreamWaitEvent(stream, join_ev, 0));
+    }
+    TOTEM_TRY(st);
     return combine_results(de, launches);
   };
 
-  if (!fused || profiling || !totem::slice_graphs_enabled()) {
+  // a graph costs its capture, and a long run of short batches has thousands of launches to spare
+  const long per_batch = 2L * slices + n_events, batches = (items_total + B - 1) / B;
+  if (!fused || profiling || !totem::slice_graphs_enabled() || per_batch * batches > 8192) {
     TOTEM_TRY(enqueue());
   } else {
     // what the launches embed: sizes, buffer addresses and the detection events
-    std::vector<long long> key = {h, items_total, B, slices, col_variant, t_storage, n_events, exit_event, aper_num,
+    std::vector<long long> key = {h, items_total, B, chains, slices, col_variant, t_storage, n_events, exit_event, aper_num,
                                   w_num, depth, nblk, L, p_h, p_w, begin_row, begin_col, step, width_red,
                                   (long long)tslice_bytes, skip_band ? 1 : 0, skip_rows ? 1 : 0, row_variant};
     for (const void* q : {(const void*)psi.p, (const void*)part.p, (const void*)acc.p, (const void*)probe.p,
@@ -1154,7 +1221,7 @@ Status totem_session::run(int what, const TotemRunOptions* opt) {
     if (h == w && totem::radix_window_ops(h)) rv = cv = 0;  // mixed-radix windows: default shapes only
     used_row_variant = rv ? rv : 1;
     used_col_variant = cv ? cv : 1;
-    TOTEM_TRY(slice_loop(o.path, batch, cv, o.t_storage, &launches, &batch_used, rv));
+    TOTEM_TRY(slice_loop(o.path, batch, o.batch > 0, cv, o.t_storage, &launches, &batch_used, rv));
   }
   else has_result = true;
   TOTEM_CUDA(cudaEventRecord(ev[2], stream));

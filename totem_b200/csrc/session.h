@@ -148,6 +148,9 @@ struct totem_session {
   int device = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
+  // second chain of the slice loop (slice_loop): forked from and joined to ``stream`` in every run
+  cudaStream_t stream2 = nullptr;
+  cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
   std::mutex mu;
 
   // request metadata
@@ -217,6 +220,9 @@ struct totem_session {
     for (auto& e : ev)
       if (e) cudaEventDestroy(e);
     for (auto& e : pev) cudaEventDestroy(e);
+    for (auto& e : {fork_ev, join_ev})
+      if (e) cudaEventDestroy(e);
+    if (stream2) cudaStreamDestroy(stream2);
     if (own_stream && stream) cudaStreamDestroy(stream);
   }
 
@@ -285,8 +291,10 @@ struct totem_session {
   // Per-event detector sums acc[event][w][A][depth] -> out_result (exit) and out_mid (layers),
   // weighted by gfsf over w (accumulate_result, cuda_source_lobato.cu:981-1015).
   Status combine_results(const totem::DetectionEvents& de, int* launches);
-  Status slice_loop(int path, int batch, int col_variant, int t_storage, int* launches, int* batch_used,
-                    int row_variant = 0);
+  // ``batch_fixed``: the caller chose the batch (one chain of such batches); otherwise it is a bound.
+  Status slice_loop(int path, int batch, bool batch_fixed, int col_variant, int t_storage, int* launches,
+                    int* batch_used, int row_variant = 0);
+  Status second_stream();
   // The transmission slices as the slice loop reads them (complex64, or bfloat16 pairs).
   Status transmission_for(int t_storage, const void** t, size_t* slice_bytes, int* launches);
   Status run_graphed(const std::vector<long long>& key, const std::function<Status()>& enqueue, int* launches);
