@@ -6,6 +6,7 @@ from __future__ import annotations
 
 import contextlib
 import ctypes as C
+from concurrent import futures
 import os
 import re
 
@@ -202,6 +203,30 @@ def _d(a):
     return np.ascontiguousarray(a, dtype=np.float64)
 
 
+def _split(z):
+    """Real and imaginary part of a complex array as two contiguous float64 arrays; large ones are
+    copied by several threads (the copies release the interpreter lock): 5 planes of 1024^2 in 5
+    instead of 28 ms."""
+    z = np.ascontiguousarray(z, dtype=np.complex128)
+    pair = z.reshape(-1).view(np.float64).reshape(-1, 2)
+    re_, im_ = np.empty(z.shape), np.empty(z.shape)
+    n = len(pair)
+    step = max(_SPLIT_GRAIN, -(-n // 8))
+
+    def copy(lo):
+        re_.reshape(-1)[lo:lo + step] = pair[lo:lo + step, 0]
+        im_.reshape(-1)[lo:lo + step] = pair[lo:lo + step, 1]
+    if n <= step:
+        copy(0)
+    else:
+        with futures.ThreadPoolExecutor(8) as pool:
+            list(pool.map(copy, range(0, n, step)))
+    return re_, im_
+
+
+_SPLIT_GRAIN = 1 << 17
+
+
 def _ptr(a, typ=_dp):
     if a is None:
         return C.cast(None, typ)
@@ -224,11 +249,9 @@ class Marshalled:
         a.struct_size = C.sizeof(TotemStemArgs)
         a.param = PARAM_LOBATO if req.param == "l" else PARAM_PENG
         if stem:
-            a.probe_re = _ptr(k(req.probe.real))
-            a.probe_im = _ptr(k(req.probe.imag))
+            a.probe_re, a.probe_im = (_ptr(k(v)) for v in _split(req.probe))
             a.aper = _ptr(k(req.aper))
-            a.prop_re = _ptr(k(req.prop.real))
-            a.prop_im = _ptr(k(req.prop.imag))
+            a.prop_re, a.prop_im = (_ptr(k(v)) for v in _split(req.prop))
             a.gfsf = _ptr(k(req.gfsf))
             a.aper2 = _ptr(k(req.aper2))
             a.height, a.width = req.height, req.width
@@ -429,19 +452,21 @@ class _HrtemMarshalled:
     def __init__(self, spec, t_storage):
         self.keep = []
 
-        def k(a):
-            a = np.ascontiguousarray(a, dtype=np.float64)
-            self.keep.append(a)
-            return _ptr(a)
+        def k(z):
+            pair = _split(z)
+            self.keep.extend(pair)
+            return (_ptr(v) for v in pair)
         a = TotemHrtemArgs()
         a.struct_size = C.sizeof(TotemHrtemArgs)
         if spec.wave is not None:
-            a.wave_re, a.wave_im = k(spec.wave.real), k(spec.wave.imag)
-        a.prop_re, a.prop_im = k(spec.prop.real), k(spec.prop.imag)
+            a.wave_re, a.wave_im = k(spec.wave)
+        a.prop_re, a.prop_im = k(spec.prop)
         if spec.tf is not None and len(spec.tf):
             a.defoci = len(spec.tf)
-            a.tf_re, a.tf_im = k(spec.tf.real), k(spec.tf.imag)
-            a.weights = k(spec.weights)
+            a.tf_re, a.tf_im = k(spec.tf)
+            weights = _d(spec.weights)
+            self.keep.append(weights)
+            a.weights = _ptr(weights)
         a.t_storage = t_storage
         self.args = a
 
@@ -458,7 +483,11 @@ def _hrtem_marshal(spec, ph, pw, t_storage, exit_wave, image):
         out.image = _ptr(img)
 
     def ex():
-        return None if ere is None else ere + 1j * eim
+        if ere is None:
+            return None
+        wave = np.empty((ph, pw), dtype=np.complex128)
+        wave.real, wave.imag = ere, eim
+        return wave
     return h, out, ex, img
 
 

@@ -184,15 +184,16 @@ std::vector<float2> stage_twiddles(int n);
 // ---------------------------------------------------------------------------------------------
 // Fused multislice
 // ---------------------------------------------------------------------------------------------
-// Spectral band of a propagator H [N][N] (FFT order): the largest index distance from DC,
-// min(c, N - c), of a column holding a non-zero entry.  The columns c with band < c < N - band are
-// zero in every row, so after the column pass's multiply by H those columns of the wave are zero
-// whatever the wave was.  The reference's propagator is cut at 2/3 of Nyquist
-// (ToTEM_submit_v1.m:1558-1564): band = N / 3.
-int spectral_band(const double* re, const double* im, int h, int w);
-// The same for rows: the largest index distance from DC of a row holding a non-zero entry, and
-// whether an n x n window's passes may take its rows BandRows<n> (fft.cuh) as zero.
-int spectral_row_band(const double* re, const double* im, int h, int w);
+// Spectral band of a propagator H [N][N] (FFT order): ``cols`` the largest index distance from DC,
+// min(c, N - c), of a column holding a non-zero entry, ``rows`` that of a row.  The columns c with
+// cols < c < N - cols are zero in every row, so after the column pass's multiply by H those columns of
+// the wave are zero whatever the wave was; likewise the rows.  The reference's propagator is cut at
+// 2/3 of Nyquist (ToTEM_submit_v1.m:1558-1564): N / 3 for both.
+struct SpectralBand {
+  int cols, rows;
+};
+SpectralBand spectral_band(const double* re, const double* im, int h, int w);
+// Whether an n x n window's passes may take its rows BandRows<n> (fft.cuh) as zero.
 bool band_rows_ok(int n, int row_band);
 // Column tiles [z0, z0 + nskip) left out of a column-pass launch.
 struct TileSkip {
@@ -348,6 +349,8 @@ Status launch_plain_tf_mul(float2* work, const float2* spec, const float2* tf, i
 Status launch_plain_image(const float2* work, int planes, const double* w, float s, int vol, float* out,
                           cudaStream_t st);
 // CBED: out[h][w] = sum_q gfsf[q] |fftshift(spec_q)|^2 over w_num kept spectra [w_num][h][w] (FP64).
+// out[i] = 1 (complex64): the plane incident wave of HRTEM.
+Status launch_fill_ones(float2* out, long n, cudaStream_t st);
 Status launch_cbed_pattern(const float2* spec, const double* gfsf, int w_num, int h, int w, double* out,
                            cudaStream_t st);
 Status launch_plain_detect(const float2* psi, const float* masks, int aper_num, int vol, int items,

@@ -366,20 +366,26 @@ Status totem_session::upload_args(const TotemStemArgs* a, bool stem) {
     host_cn = split_rows(a->ele_n_corr, n_corr, 5, nullptr, beg_cn);
     host_ci = split_rows(a->ele_n_i_corr, n_corr_i, 8, nullptr, beg_ci);
     const size_t plane = (size_t)p_h * p_w;
-    std::vector<float> c(plane * cim_len);
-    for (size_t i = 0; i < c.size(); ++i) c[i] = (float)a->corr_info_matrix[i];
-    TOTEM_TRY(upload(cim, c, st));
+    TOTEM_TRY(totem::upload_f32(cim, a->corr_info_matrix, plane * cim_len, st));
   }
 
   // reciprocal grids: detect the reference's separable meshgrid layout
   const size_t plane = (size_t)p_h * p_w;
-  separable = true;
-  for (int r = 0; r < p_h && separable; ++r)
-    for (int c = 0; c < p_w; ++c)
-      if (a->kx[(size_t)r * p_w + c] != a->kx[c] || a->ky[(size_t)r * p_w + c] != a->ky[(size_t)r * p_w]) {
-        separable = false;
-        break;
+  std::atomic<bool> meshgrid{true}, ones{true};
+  totem::host_parallel(p_h, totem::kHostGrain / p_w + 1, [&](size_t lo, size_t hi) {
+    bool mesh = true, one = true;
+    for (size_t r = lo; r < hi && (mesh || one); ++r) {
+      const double *kx = a->kx + r * p_w, *ky = a->ky + r * p_w, *ap = a->aper_true + r * p_w;
+      for (int c = 0; c < p_w; ++c) {
+        mesh &= kx[c] == a->kx[c] && ky[c] == ky[0];
+        one &= ap[c] == 1.0;
       }
+    }
+    if (!mesh) meshgrid = false;
+    if (!one) ones = false;
+  });
+  separable = meshgrid;
+  aper_true_ones = ones;
   // neutral, ionic and correction rows: by species on separable grids (k_tx_species or
   // gridding), row by row otherwise
   grid_ok = false;
@@ -409,9 +415,7 @@ Status totem_session::upload_args(const TotemStemArgs* a, bool stem) {
     TOTEM_TRY(rows_cn.put(host_cn, st));
     TOTEM_TRY(rows_ci.put(host_ci, st));
   }
-  std::vector<float> s2f(plane);
-  for (size_t i = 0; i < plane; ++i) s2f[i] = (float)a->s_2[i];
-  TOTEM_TRY(upload(s2, s2f, st));
+  TOTEM_TRY(totem::upload_f32(s2, a->s_2, plane, st));
   if (separable) {
     std::vector<double> kxa(a->kx, a->kx + p_w), kya(p_h);
     for (int r = 0; r < p_h; ++r) kya[r] = a->ky[(size_t)r * p_w];
@@ -421,43 +425,37 @@ Status totem_session::upload_args(const TotemStemArgs* a, bool stem) {
     TOTEM_TRY(upload(kx, std::vector<double>(a->kx, a->kx + plane), st));
     TOTEM_TRY(upload(ky, std::vector<double>(a->ky, a->ky + plane), st));
   }
-  aper_true_ones = true;
-  for (size_t i = 0; i < plane; ++i)
-    if (a->aper_true[i] != 1.0) {
-      aper_true_ones = false;
-      break;
-    }
-  if (!aper_true_ones) {
-    std::vector<float> at(plane);
-    for (size_t i = 0; i < plane; ++i) at[i] = (float)a->aper_true[i];
-    TOTEM_TRY(upload(aper_true, at, st));
-  }
+  if (!aper_true_ones) TOTEM_TRY(totem::upload_f32(aper_true, a->aper_true, plane, st));
   TOTEM_TRY(upload(tw_pw, twiddles(p_w), st));
   TOTEM_TRY(upload(tw_ph, twiddles(p_h), st));
 
   // probe, propagator, masks
   if (want_stem) {
     const size_t vol = (size_t)h * w;
-    std::vector<float2> pr(vol * w_num), hp(vol);
-    for (size_t i = 0; i < pr.size(); ++i) pr[i] = make_float2((float)a->probe_re[i], (float)a->probe_im[i]);
-    for (size_t i = 0; i < vol; ++i) hp[i] = make_float2((float)a->prop_re[i], (float)a->prop_im[i]);
-    TOTEM_TRY(upload(probe, pr, st));
-    TOTEM_TRY(upload(prop, hp, st));
-    band = (h == w) ? totem::spectral_band(a->prop_re, a->prop_im, h, w) : (1 << 30);
-    row_band = (h == w) ? totem::spectral_row_band(a->prop_re, a->prop_im, h, w) : (1 << 30);
+    TOTEM_TRY(totem::upload_c64(probe, a->probe_re, a->probe_im, vol * w_num, st));
+    TOTEM_TRY(totem::upload_c64(prop, a->prop_re, a->prop_im, vol, st));
+    totem::SpectralBand b{1 << 30, 1 << 30};
+    if (h == w) b = totem::spectral_band(a->prop_re, a->prop_im, h, w);
+    band = b.cols;
+    row_band = b.rows;
     // exit detector: ifftshift(aper) (the reference shifts the wave instead, cuda_source_lobato.cu:1415)
-    std::vector<float> me(vol * std::max(aper_num, 1)), mm;
-    for (int q = 0; q < aper_num; ++q)
-      for (int r = 0; r < h; ++r)
-        for (int c = 0; c < w; ++c)
-          me[(size_t)q * vol + (size_t)r * w + c] =
-              (float)a->aper[(size_t)q * vol + (size_t)((r + h / 2) % h) * w + (c + w / 2) % w];
-    TOTEM_TRY(upload(mask_exit, me, st));
-    if (a->layer_len > 0 && aper_num > 0) {
-      mm.resize(vol * aper_num);
-      for (size_t i = 0; i < mm.size(); ++i) mm[i] = (float)a->aper2[i];
-      TOTEM_TRY(upload(mask_mid, mm, st));
-    }
+    totem::HostArray<float> me(vol * std::max(aper_num, 1));
+    if (aper_num == 0) std::fill(me.data(), me.data() + vol, 0.f);
+    totem::host_parallel((size_t)aper_num * h, totem::kHostGrain / w + 1, [&](size_t lo, size_t hi) {
+      for (size_t q = lo; q < hi; ++q) {  // row q % h of mask q / h, from the row h / 2 further on
+        const double* src = a->aper + q / h * vol + (q % h + h / 2) % h * (size_t)w;
+        float* dst = me.data() + q * w;
+        for (int c = 0; c < w / 2; ++c) {
+          dst[c] = (float)src[c + w / 2];
+          dst[c + w / 2] = (float)src[c];
+        }
+      }
+    });
+    const size_t mask_bytes = vol * std::max(aper_num, 1) * sizeof(float);
+    TOTEM_TRY(mask_exit.ensure(mask_bytes));
+    TOTEM_CUDA(cudaMemcpyAsync(mask_exit.p, me.data(), mask_bytes, cudaMemcpyHostToDevice, st));
+    g_h2d_bytes += (long long)mask_bytes;
+    if (a->layer_len > 0 && aper_num > 0) TOTEM_TRY(totem::upload_f32(mask_mid, a->aper2, vol * aper_num, st));
     if (h == w) TOTEM_TRY(upload(tw_n, twiddles(h), st));
     TOTEM_TRY(upload(gfsf_d, gfsf, st));
   }
@@ -995,13 +993,13 @@ Status totem_session::hrtem(const TotemHrtemArgs* hr, TotemHrtemOut* out) {
   size_t tslice_bytes = 0;
   TOTEM_TRY(transmission_for(hr->t_storage, &Tslices, &tslice_bytes, &launches));
 
-  std::vector<float2> wave(vol), prop(vol);
-  for (size_t i = 0; i < vol; ++i) {
-    wave[i] = hr->wave_re ? make_float2((float)hr->wave_re[i], (float)hr->wave_im[i]) : make_float2(1.f, 0.f);
-    prop[i] = make_float2((float)hr->prop_re[i], (float)hr->prop_im[i]);
+  if (hr->wave_re) {
+    TOTEM_TRY(totem::upload_c64(hr_wave, hr->wave_re, hr->wave_im, vol, stream));
+  } else {
+    TOTEM_TRY(hr_wave.ensure(vol * sizeof(float2)));
+    TOTEM_TRY(totem::launch_fill_ones(hr_wave.as<float2>(), (long)vol, stream));
   }
-  TOTEM_TRY(upload(hr_wave, wave, stream));
-  TOTEM_TRY(upload(hr_prop, prop, stream));
+  TOTEM_TRY(totem::upload_c64(hr_prop, hr->prop_re, hr->prop_im, vol, stream));
   TOTEM_TRY(psi.ensure(vol * sizeof(float2)));
   timing.slice_path = fused ? TOTEM_PATH_FUSED : TOTEM_PATH_PLAIN;
   timing.tx_fft_path = ran_tx_fft;
@@ -1018,14 +1016,11 @@ Status totem_session::hrtem(const TotemHrtemArgs* hr, TotemHrtemOut* out) {
   s.t_bf16 = (hr->t_storage == TOTEM_T_BF16);
   // every pass leaves out the propagator's zero band (the last column pass writes zeros there
   // into the kept spectrum); the bfloat16 trial computes every column
-  s.skip_band = (totem::band_skip_enabled() && hr->t_storage == TOTEM_T_COMPLEX64 &&
-                 totem::band_skip_ok(n, totem::spectral_band(hr->prop_re, hr->prop_im, n, n), 0))
-                    ? 1
-                    : 0;
-  s.skip_rows = (totem::band_skip_enabled() && hr->t_storage == TOTEM_T_COMPLEX64 &&
-                 totem::band_rows_ok(n, totem::spectral_row_band(hr->prop_re, hr->prop_im, n, n)))
-                    ? 1
-                    : 0;
+  if (totem::band_skip_enabled() && hr->t_storage == TOTEM_T_COMPLEX64) {
+    const totem::SpectralBand b = totem::spectral_band(hr->prop_re, hr->prop_im, n, n);
+    s.skip_band = totem::band_skip_ok(n, b.cols, 0) ? 1 : 0;
+    s.skip_rows = totem::band_rows_ok(n, b.rows) ? 1 : 0;
+  }
   auto tslice = [&](int k) { return static_cast<const char*>(Tslices) + (size_t)k * tslice_bytes; };
   // psi = wave .* T_0, then per slice FFT2 .* psf_fft IFFT2 .* T_{k+1}; the last column pass keeps
   // the spectrum FFT2(psi_{S-1} .* T) .* psf_fft, whose IFFT2 is the exit wave
@@ -1037,34 +1032,33 @@ Status totem_session::hrtem(const TotemHrtemArgs* hr, TotemHrtemOut* out) {
   const float2* spec = psi.as<float2>();
   const bool want_exit = out && (out->exit_re || out->exit_im);
   const bool want_img = out && out->image && hr->defoci > 0;
-  std::vector<float2> exit_h;
-  std::vector<float> img_h;
+  totem::HostArray<float2> exit_h(want_exit ? vol : 0);
+  totem::HostArray<float> img_h(want_img ? vol : 0);
   if (want_exit) {
     TOTEM_TRY(hr_work.ensure(vol * sizeof(float2)));
     TOTEM_TRY(hr_exit.ensure(vol * sizeof(float2)));
     TOTEM_TRY(totem::launch_exit_wave(n, spec, hr_work.as<float2>(), hr_exit.as<float2>(), tw_pw.as<float2>(), stream));
-    exit_h.resize(vol);
     TOTEM_CUDA(cudaMemcpyAsync(exit_h.data(), hr_exit.p, vol * sizeof(float2), cudaMemcpyDeviceToHost, stream));
   }
   if (want_img) {
     const int K = hr->defoci;
-    std::vector<float2> tf((size_t)K * vol);
-    for (size_t i = 0; i < tf.size(); ++i) tf[i] = make_float2((float)hr->tf_re[i], (float)hr->tf_im[i]);
-    TOTEM_TRY(upload(hr_tf, tf, stream));
+    TOTEM_TRY(totem::upload_c64(hr_tf, hr->tf_re, hr->tf_im, (size_t)K * vol, stream));
     TOTEM_TRY(upload(hr_w, std::vector<double>(hr->weights, hr->weights + K), stream));
     TOTEM_TRY(hr_work.ensure((size_t)K * vol * sizeof(float2)));
     TOTEM_TRY(hr_img.ensure(vol * sizeof(float)));
     TOTEM_TRY(totem::launch_tcc_image(n, spec, hr_tf.as<float2>(), K, hr_w.as<double>(), hr_work.as<float2>(),
                                       hr_img.as<float>(), tw_pw.as<float2>(), stream));
-    img_h.resize(vol);
     TOTEM_CUDA(cudaMemcpyAsync(img_h.data(), hr_img.p, vol * sizeof(float), cudaMemcpyDeviceToHost, stream));
   }
   TOTEM_CUDA(cudaStreamSynchronize(stream));
-  for (size_t i = 0; i < exit_h.size(); ++i) {
-    if (out->exit_re) out->exit_re[i] = exit_h[i].x;
-    if (out->exit_im) out->exit_im[i] = exit_h[i].y;
-  }
-  for (size_t i = 0; i < img_h.size(); ++i) out->image[i] = img_h[i];
+  totem::host_parallel(vol, totem::kHostGrain, [&](size_t lo, size_t hi) {
+    if (want_exit && out->exit_re)
+      for (size_t i = lo; i < hi; ++i) out->exit_re[i] = exit_h[i].x;
+    if (want_exit && out->exit_im)
+      for (size_t i = lo; i < hi; ++i) out->exit_im[i] = exit_h[i].y;
+    if (want_img)
+      for (size_t i = lo; i < hi; ++i) out->image[i] = img_h[i];
+  });
   return Status::Ok();
 }
 
@@ -1092,21 +1086,18 @@ Status totem_session::hrtem_plain(const TotemHrtemArgs* hr, TotemHrtemOut* out, 
   const float scale = 1.f / ((float)n * (float)n);
   const bool want_exit = out && (out->exit_re || out->exit_im);
   const bool want_img = out && out->image && hr->defoci > 0;
-  std::vector<float2> exit_h;
-  std::vector<float> img_h;
+  totem::HostArray<float2> exit_h(want_exit ? vol : 0);
+  totem::HostArray<float> img_h(want_img ? vol : 0);
   if (want_exit) {
     TOTEM_TRY(hr_exit.ensure(vol * sizeof(float2)));
     TOTEM_CUDA(cudaMemcpyAsync(hr_exit.p, ps, vol * sizeof(float2), cudaMemcpyDeviceToDevice, stream));
     TOTEM_CUFFT(cufftExecC2C(one, (cufftComplex*)hr_exit.p, (cufftComplex*)hr_exit.p, CUFFT_INVERSE));
     TOTEM_TRY(totem::launch_plain_scale(hr_exit.as<float2>(), scale, (long)vol, stream));
-    exit_h.resize(vol);
     TOTEM_CUDA(cudaMemcpyAsync(exit_h.data(), hr_exit.p, vol * sizeof(float2), cudaMemcpyDeviceToHost, stream));
   }
   if (want_img) {
     const int K = hr->defoci;
-    std::vector<float2> tf((size_t)K * vol);
-    for (size_t i = 0; i < tf.size(); ++i) tf[i] = make_float2((float)hr->tf_re[i], (float)hr->tf_im[i]);
-    TOTEM_TRY(upload(hr_tf, tf, stream));
+    TOTEM_TRY(totem::upload_c64(hr_tf, hr->tf_re, hr->tf_im, (size_t)K * vol, stream));
     TOTEM_TRY(upload(hr_w, std::vector<double>(hr->weights, hr->weights + K), stream));
     TOTEM_TRY(hr_work.ensure((size_t)K * vol * sizeof(float2)));
     TOTEM_TRY(hr_img.ensure(vol * sizeof(float)));
@@ -1116,15 +1107,17 @@ Status totem_session::hrtem_plain(const TotemHrtemArgs* hr, TotemHrtemOut* out, 
     TOTEM_CUFFT(cufftExecC2C(planes, (cufftComplex*)hr_work.p, (cufftComplex*)hr_work.p, CUFFT_INVERSE));
     TOTEM_TRY(totem::launch_plain_image(hr_work.as<float2>(), K, hr_w.as<double>(), scale, (int)vol,
                                         hr_img.as<float>(), stream));
-    img_h.resize(vol);
     TOTEM_CUDA(cudaMemcpyAsync(img_h.data(), hr_img.p, vol * sizeof(float), cudaMemcpyDeviceToHost, stream));
   }
   TOTEM_CUDA(cudaStreamSynchronize(stream));
-  for (size_t i = 0; i < exit_h.size(); ++i) {
-    if (out->exit_re) out->exit_re[i] = exit_h[i].x;
-    if (out->exit_im) out->exit_im[i] = exit_h[i].y;
-  }
-  for (size_t i = 0; i < img_h.size(); ++i) out->image[i] = img_h[i];
+  totem::host_parallel(vol, totem::kHostGrain, [&](size_t lo, size_t hi) {
+    if (want_exit && out->exit_re)
+      for (size_t i = lo; i < hi; ++i) out->exit_re[i] = exit_h[i].x;
+    if (want_exit && out->exit_im)
+      for (size_t i = lo; i < hi; ++i) out->exit_im[i] = exit_h[i].y;
+    if (want_img)
+      for (size_t i = lo; i < hi; ++i) out->image[i] = img_h[i];
+  });
   return Status::Ok();
 }
 
@@ -1281,13 +1274,15 @@ Status totem_session::download(TotemStemOut* out) {
   }
   if ((out->potential_re || out->potential_im) && t_valid && slices > 0) {
     const size_t n = (size_t)p_h * p_w * slices;
-    std::vector<float2> t(n);
+    totem::HostArray<float2> t(n);
     TOTEM_CUDA(cudaMemcpy(t.data(), T.p, n * sizeof(float2), cudaMemcpyDeviceToHost));
     d2h += (long long)(n * sizeof(float2));
-    for (size_t i = 0; i < n; ++i) {
-      if (out->potential_re) out->potential_re[i] = t[i].x;
-      if (out->potential_im) out->potential_im[i] = t[i].y;
-    }
+    totem::host_parallel(n, totem::kHostGrain, [&](size_t lo, size_t hi) {
+      for (size_t i = lo; i < hi; ++i) {
+        if (out->potential_re) out->potential_re[i] = t[i].x;
+        if (out->potential_im) out->potential_im[i] = t[i].y;
+      }
+    });
   }
   d2h_bytes = d2h;
   timing.d2h_bytes = d2h;

@@ -14,6 +14,9 @@
 // Layout in HBM: psi[item][row][col] complex64, item = w * depth + pos (probe-major, as the
 // reference's w_series loop); T[slice][P_H][P_W]; H[N][N] and the masks [A][N][N] in natural
 // FFT order (the masks for the exit detector are ifftshift(aper), computed at upload).
+#include <mutex>
+
+#include "host_parallel.h"
 #include "passes.cuh"
 
 namespace totem {
@@ -146,31 +149,30 @@ TileSkip band_tiles(int n, int nblk) {
   return t;
 }
 
-int spectral_band(const double* re, const double* im, int h, int w) {
-  int band = 0;
-  for (int c = 0; c < w; ++c) {
-    const int dist = c < w - c ? c : w - c;
-    if (dist <= band) continue;
-    for (int r = 0; r < h; ++r)
-      if (re[(size_t)r * w + c] != 0.0 || im[(size_t)r * w + c] != 0.0) {
-        band = dist;
-        break;
-      }
-  }
-  return band;
-}
-
-int spectral_row_band(const double* re, const double* im, int h, int w) {
-  int band = 0;
-  for (int r = 0; r < h; ++r) {
-    const int dist = r < h - r ? r : h - r;
-    if (dist <= band) continue;
-    for (int c = 0; c < w; ++c)
-      if (re[(size_t)r * w + c] != 0.0 || im[(size_t)r * w + c] != 0.0) {
-        band = dist;
-        break;
-      }
-  }
+SpectralBand spectral_band(const double* re, const double* im, int h, int w) {
+  // each thread a range of rows; within a row only the columns beyond the largest distance it has
+  // found so far, and those within it where the row itself is beyond the largest row distance
+  std::mutex mu;
+  SpectralBand band{0, 0};
+  host_parallel(h, (1 << 16) / std::max(w, 1) + 1, [&](size_t lo, size_t hi) {
+    int cols = 0, rows = 0;
+    for (int r = (int)lo; r < (int)hi; ++r) {
+      const double *pr = re + (size_t)r * w, *pi = im + (size_t)r * w;
+      bool any = false;
+      for (int c = cols + 1; c < w - cols; ++c)
+        if (pr[c] != 0.0 || pi[c] != 0.0) {
+          any = true;
+          cols = std::max(cols, std::min(c, w - c));
+        }
+      const int dist = std::min(r, h - r);
+      if (dist <= rows) continue;
+      for (int c = 0; c < w && !any; ++c) any = pr[c] != 0.0 || pi[c] != 0.0;
+      if (any) rows = dist;
+    }
+    std::lock_guard<std::mutex> lk(mu);
+    band.cols = std::max(band.cols, cols);
+    band.rows = std::max(band.rows, rows);
+  });
   return band;
 }
 

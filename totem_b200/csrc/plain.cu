@@ -116,6 +116,11 @@ __global__ void k_cbed_pattern(const float2* __restrict__ spec, const double* __
   }
 }
 
+__global__ void k_fill_ones(float2* __restrict__ out, long n) {
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+    out[i] = make_float2(1.f, 0.f);
+}
+
 inline int grid_for(long total) { return (int)std::min<long>((total + 255) / 256, 148L * 32); }
 
 }  // namespace
@@ -165,6 +170,12 @@ Status launch_plain_image(const float2* work, int planes, const double* w, float
   if (vol == 0) return Status::Ok();
   k_plain_image<<<grid_for(vol), 256, 0, st>>>(work, planes, w, s, vol, out);
   return cuda_status(cudaGetLastError(), "k_plain_image");
+}
+
+Status launch_fill_ones(float2* out, long n, cudaStream_t st) {
+  if (n == 0) return Status::Ok();
+  k_fill_ones<<<grid_for(n), 256, 0, st>>>(out, n);
+  return cuda_status(cudaGetLastError(), "k_fill_ones");
 }
 
 Status launch_cbed_pattern(const float2* spec, const double* gfsf, int w_num, int h, int w, double* out,

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "host_parallel.h"
 
 namespace totem {
 
@@ -54,6 +55,44 @@ Status upload(DevBuf& b, const std::vector<T>& v, cudaStream_t st) {
   TOTEM_TRY(b.ensure(v.size() * sizeof(T)));
   if (!v.empty()) TOTEM_CUDA(cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st));
   g_h2d_bytes += (long long)(v.size() * sizeof(T));
+  return Status::Ok();
+}
+
+// Elements a host thread should have to itself: below half a million the threads' start, on a busy
+// host, costs more than the loop.
+constexpr size_t kHostGrain = 1 << 18;
+
+// The caller's FP64 array of n elements as FP32, converted by several threads.
+inline Status upload_f32(DevBuf& b, const double* v, size_t n, cudaStream_t st) {
+  TOTEM_TRY(b.ensure(n * sizeof(float)));
+  if (n == 0) return Status::Ok();
+  HostArray<float> f(n);
+  host_parallel(n, kHostGrain, [&](size_t lo, size_t hi) {
+    for (size_t i = lo; i < hi; ++i) f[i] = (float)v[i];
+  });
+  // (a copy from pageable memory returns once its source has been read)
+  TOTEM_CUDA(cudaMemcpyAsync(b.p, f.data(), n * sizeof(float), cudaMemcpyHostToDevice, st));
+  g_h2d_bytes += (long long)(n * sizeof(float));
+  return Status::Ok();
+}
+
+// re + i im of n elements as complex64, converted by several threads block by block: a block is
+// small enough to stay in the host's caches until the copy has read it, and its pages are touched
+// once instead of once per element (5 planes of 1024^2: 29 ms by one thread into a vector of the
+// whole array).
+inline Status upload_c64(DevBuf& b, const double* re, const double* im, size_t n, cudaStream_t st) {
+  constexpr size_t kBlock = 1 << 20;
+  TOTEM_TRY(b.ensure(n * sizeof(float2)));
+  HostArray<float2> f(std::min(n, kBlock));
+  for (size_t at = 0; at < n; at += kBlock) {
+    const size_t count = std::min(kBlock, n - at);
+    host_parallel(count, kHostGrain, [&](size_t lo, size_t hi) {
+      for (size_t i = lo; i < hi; ++i) f[i] = make_float2((float)re[at + i], (float)im[at + i]);
+    });
+    // (a copy from pageable memory returns once its source has been read)
+    TOTEM_CUDA(cudaMemcpyAsync(b.as<float2>() + at, f.data(), count * sizeof(float2), cudaMemcpyHostToDevice, st));
+  }
+  g_h2d_bytes += (long long)(n * sizeof(float2));
   return Status::Ok();
 }
 
@@ -200,9 +239,8 @@ struct totem_session {
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
   TotemTiming timing{};
   long long h2d_bytes = 0, d2h_bytes = 0;
-  // band of the uploaded propagator (totem::spectral_band; n / 2 and above: no zero band)
-  int band = 1 << 30;
-  int row_band = 1 << 30;  // totem::spectral_row_band
+  // bands of the uploaded propagator (totem::spectral_band; n / 2 and above: no zero band)
+  int band = 1 << 30, row_band = 1 << 30;
   // which implementations the last run used (TotemTiming.slice_path / tx_fft_path / tx_builder)
   int ran_slice_path = -1, ran_tx_fft = -1, ran_tx_builder = -1;
   int used_row_variant = 0, used_col_variant = 0;
