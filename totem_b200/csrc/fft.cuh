@@ -606,7 +606,12 @@ struct RowCfg {
 };
 // Columns: G adjacent columns per CTA, thread (j, g) = (tid / G, tid % G), so a warp's loads
 // cover 32 / G rows x G columns.
-template <int N, int CTAS128 = 4, int GW = 0>
+// resident CTAs of 128 threads a column pass asks for per SM by default: 4, a 128-register cap; the
+// 16-point transforms of 128^2 and 256^2 fit an 80-register cap without spilling, and run faster at
+// six (slice loop 0.0788 -> 0.0748 and 0.323 -> 0.294 us per probe*slice)
+template <int N>
+constexpr int col_ctas() { return (N == 128 || N == 256) ? 6 : 4; }
+template <int N, int CTAS128 = col_ctas<N>(), int GW = 0>
 struct ColCfg {
   static constexpr int P = Fft<N>::P, T = Fft<N>::T;
   // GW = 0: the default width, 16 columns (one 128-byte segment per row) up to N = 512, 8 (64
@@ -618,7 +623,6 @@ struct ColCfg {
   // slice loops; at 1600^2 the half tile (320 threads, one CTA per SM) was 8 % slower.
   static constexpr int G = GW ? GW : (((N & (N - 1)) && G0 * T > 256 && (G0 / 2) * T <= 256) ? G0 / 2 : G0);
   static_assert((G * T) % 32 == 0 && N % G == 0, "column tile: whole warps, whole tiles");
-  // resident CTAs of 128 threads requested per SM (4 = a 128-register cap)
   static constexpr int MINB = (CTAS128 * 128 / (G * T) > 0) ? CTAS128 * 128 / (G * T) : 1;
 };
 

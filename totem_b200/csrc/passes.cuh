@@ -128,7 +128,7 @@ Status col_pass(const SliceLoopArgs& a, int flags, cudaStream_t st) {
     case 3: return col_pass_v<N, false, (N <= 1024 ? 6 : 4), 0>(a, flags, st);
     case 5: return col_pass_v<N, false, 4, (N <= 2048 ? 8 : 0)>(a, flags, st);
     case 6: return col_pass_v<N, false, 4, (N <= 512 ? 32 : 0)>(a, flags, st);
-    default: return col_pass_v<N, false, 4, 0>(a, flags, st);
+    default: return col_pass_v<N, false, col_ctas<N>(), 0>(a, flags, st);
   }
 }
 

@@ -56,17 +56,30 @@ __device__ __forceinline__ void row_tile(float2* __restrict__ psi_item, const vo
   float2* prow = psi_item + (long)row * N;
   const RowLayout<N> L;
   const auto sync = group_sync<N>(g);
-  // The transmission window row is copied asynchronously into this row's exchange region as soon
-  // as the region is free (kernel start for the first pass, after the inverse transform's last
-  // exchange otherwise), so its latency overlaps the transform.  Each thread copies and later
-  // reads only its own elements.
+  // The transmission window row.  From N = 256 on its elements are loaded straight into registers
+  // where they are used: the copy through shared memory (below, for the shorter transforms) cost a
+  // sixth of the pass's L1 data traffic, more than the loads' latency that it hid (slice loop, us per
+  // probe*slice, copied / direct: 128^2 0.0787 / 0.0796, 256^2 0.302 / 0.294, 512^2 1.247 / 1.188,
+  // 1024^2 5.88 / 5.53, 2048^2 38.3 / 37.8).
+  // Copied: asynchronously into this row's exchange region as soon as the region is free (kernel
+  // start for the first pass, after the inverse transform's last exchange otherwise); each thread
+  // copies and later reads only its own elements.
+  constexpr bool COPY = N < 256;
   auto prefetch_t = [&]() {
+    if constexpr (COPY) {
 #pragma unroll
-    for (int m = 0; m < P; ++m) {
-      if constexpr (TB16) cp_async4(&s_x[L.pos(g, j, m)], trow + j + m * T);
-      else cp_async8(&s_x[L.pos(g, j, m)], trow + j + m * T);
+      for (int m = 0; m < P; ++m) {
+        if constexpr (TB16) cp_async4(&s_x[L.pos(g, j, m)], trow + j + m * T);
+        else cp_async8(&s_x[L.pos(g, j, m)], trow + j + m * T);
+      }
+      cp_async_commit();
     }
-    cp_async_commit();
+  };
+  auto window = [&](int m) {
+    if constexpr (COPY && TB16) return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&s_x[L.pos(g, j, m)]));
+    else if constexpr (COPY) return s_x[L.pos(g, j, m)];
+    else if constexpr (TB16) return __bfloat1622float2(trow[j + m * T]);
+    else return __ldg(trow + j + m * T);
   };
   float2 v[P];
   if (FIRST) {
@@ -80,15 +93,10 @@ __device__ __forceinline__ void row_tile(float2* __restrict__ psi_item, const vo
   }
   __syncthreads();  // twiddles staged
   if (!FIRST) fft_regs<N, true, SKIP ? mlo : 0, SKIP ? mhi : 0>(v, j, g, s_tw, s_x, L, sync, prefetch_t);
-  cp_async_wait_all();
+  if constexpr (COPY) cp_async_wait_all();
 #pragma unroll
-  for (int m = 0; m < P; ++m) {
-    float2 t;
-    if constexpr (TB16) t = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&s_x[L.pos(g, j, m)]));
-    else t = s_x[L.pos(g, j, m)];
-    v[m] = cscale(cmul(v[m], t), scale);
-  }
-  sync();  // every thread of the transform has read its window values before the region is reused
+  for (int m = 0; m < P; ++m) v[m] = cscale(cmul(v[m], window(m)), scale);
+  if constexpr (COPY) sync();  // every thread of the transform has read its window values before the region is reused
   fft_regs<N, false>(v, j, g, s_tw, s_x, L, sync);
 #pragma unroll
   for (int m = 0; m < P; ++m)
