@@ -659,17 +659,18 @@ namespace {
 // streams.  Two chains of batches whose waves stay in L2 together run faster than one launch over
 // all items streaming 4 GiB through HBM: each pass finds its waves in L2, and the partial last wave
 // of CTAs of one chain's short launch is filled by the other's.  (One chain of L2-sized batches is
-// slower than either: 1.38-1.44 us.)  Measured per probe*slice, one batch against two chains:
-// 128^2 0.0901 / 0.0786, 256^2 0.323 / 0.303, 400^2 1.150 / 1.060, 512^2 1.312 / 1.247, 640^2 3.654 /
-// 3.662, 800^2 6.345 / 6.344, 1280^2 16.77 / 16.11, 2048^2 39.88 / 38.31 us.
+// slower than either: 1.38-1.44 us at 512^2.)  Measured per probe*slice, one batch against two
+// chains: 128^2 0.0838 / 0.0748, 256^2 0.328 / 0.297, 400^2 1.085 / 1.013, 512^2 1.266 / 1.187, 640^2
+// 3.514 / 3.530, 800^2 6.009 / 6.075, 1024^2 5.62-5.97 (from run to run) / 5.57, 1280^2 16.23 / 15.76,
+// 2048^2 38.44 / 36.98 us.
 //  * Waves of both chains together: 50 MB up to 576^2, 32 MB above (512^2 at 32 / 44 / 56 / 68 MB:
 //    1.291 / 1.253 / 1.247 / 1.253; 640^2 3.662 / 3.716 / 3.904 / 4.071).  Windows of which L2 does
 //    not hold two (2048^2) still gain from the overlap; eight a batch was best.
-//  * 1024^2 and 1536^2 windows stream faster than they run from L2 (5.96 against 6.30 us, 22.89
-//    against 23.70): one batch, unless there are too few to amortise it (1024^2: 8 / 16 / 30 items in
-//    one batch 6.63 / 6.82 / 6.41).
+//  * 1536^2 windows stream faster than they run from L2 (21.86 against 22.70 us; a launch over one
+//    or two of them is barely a wave of CTAs): one batch, once there are enough to amortise it.
 //  * Below 1.5 M points in all, one launch does not fill the GPU and two only add launches (256^2, 8
-//    items 1.109 / 1.142, 16 items 0.722 / 0.715; 512^2, 4 items 3.39 / 3.34, 8 items 2.47 / 2.31).
+//    items 1.084 / 1.142, 16 items 0.708 / 0.715, 64 items 0.397 / 0.321; 512^2, 4 items 3.22 / 3.34,
+//    8 items 2.39 / 2.25).
 // ``cap`` bounds the probes of a batch (0: 4 GiB of waves).
 struct SlicePlan {
   int chains = 1, batch = 1;
@@ -679,15 +680,18 @@ SlicePlan plan_chains(int n, long items, long cap) {
   if (cap <= 0) cap = std::max<long>(1, (long)((4ull << 30) / (size_t)wave));
   SlicePlan p;
   long b = std::min(cap, items);
-  const bool streams = (n == 1024 || n == 1536) && items * wave >= 0.35e9;
+  const bool streams = n == 1536 && items * wave >= 0.35e9;
   if (items >= 2 && (double)items * n * n >= 1.5 * 1048576 && !streams) {
     const double in_l2 = (n <= 576 ? 25e6 : 16e6) / (wave * 2 / 3);  // a third of the columns are left out
     p.chains = 2;
     b = std::min(std::min(cap, (items + 1) / 2), in_l2 < 0.8 ? 8 : std::max<long>(1, std::lround(in_l2)));
   }
-  long nb = (items + b - 1) / b;           // spread the items evenly over the batches,
-  if (p.chains == 2) nb += nb & 1;         // and the batches over the chains
-  p.batch = (int)((items + nb - 1) / nb);
+  long nb = (items + b - 1) / b;
+  if (p.chains == 2) {  // as many batches in either chain: the even number nearest to items / b
+    nb = 2 * std::max<long>(1, std::lround(0.5 * items / b));
+    if ((items + nb - 1) / nb > cap) nb = (items + cap - 1) / cap;
+  }
+  p.batch = (int)((items + nb - 1) / nb);  // the items spread evenly
   return p;
 }
 }  // namespace
