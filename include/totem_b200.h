@@ -202,11 +202,11 @@ TOTEM_API int totem_transmission_run(const TotemStemArgs *args, TotemStemOut *ou
  *   TOTEM_TX_DIRECT    per-species sums over atoms at every pixel: O(atoms x pixels)
  *   TOTEM_TX_GRIDDING  gridding along y onto a twice-finer axis and FFTs (a non-uniform FFT), the
  *                      x phases direct: O(atoms x width + pixels log pixels), relative error
- *                      ~1e-7; used where the axes are uniform and the height is an edge of the
- *                      fused transforms (64 to 4096, a power of two or a mixed-radix edge),
- *                      otherwise DIRECT is used.
+ *                      ~1e-7; used where the axes are uniform and the grid has at most 4096
+ *                      rows, otherwise DIRECT is used.
  * ``scratch_bytes`` bounds the gridding work memory taken during a build (0 = 1 GiB); the arrays of
- * one species of one slice (at most 64 bytes per potential pixel) are always taken. */
+ * one species of one slice (at most 64 bytes per pixel of the grid, its height rounded up to an edge of the
+ * fused transforms) are always taken. */
 #define TOTEM_TX_AUTO 0
 #define TOTEM_TX_DIRECT 1
 #define TOTEM_TX_GRIDDING 2

@@ -66,6 +66,14 @@ def _both(req, scratch):
     (2048, 64, 300, {"flag": "l"}, 0),
     (4096, 64, 40, {"centred": False, "slices": 1}, 1),
     (1600, 64, 40, {}, 0),
+    # heights that are no transform length: the next longer one spreads and transforms
+    (62, 64, 9, {}, 0),
+    (66, 80, 40, {"flag": "l"}, 0),
+    (94, 96, 33, {"centred": False}, 1),
+    (98, 64, 60, {"equal_y": True}, 0),
+    (700, 70, 64, {}, 0),
+    (1026, 64, 33, {"centred": False}, 0),
+    (4094, 64, 20, {"slices": 1}, 0),
 ])
 def test_gridding_equals_direct_sums(engine_lib, p_h, p_w, atoms, kw, scratch):
     direct, grid = _both(_request(p_h, p_w, atoms, **kw), scratch)

@@ -105,15 +105,17 @@ Status launch_tx_structure(const TxGrid& g, const AtomRowsDev& neutral, const At
 // species (no exponential per atom and pixel), then the form factor once per species and pixel.
 // Overwrites out.
 Status launch_tx_species(const TxGrid& g, const SpeciesSet& sp, float2* out, cudaStream_t st);
-// The same sums by gridding along y (tx_grid.cuh) on separable grids with a uniform ky axis and a
-// height the fused transforms take.  Work is grouped in jobs, one per (slice, kind, species)
+// The same sums by gridding along y (tx_grid.cuh) on separable grids with a uniform ky axis, up to
+// 4096 rows.  Work is grouped in jobs, one per (slice, kind, species)
 // segment, ordered by slice; a batch runs the jobs [j_lo, j_hi) in scratch memory and writes slices
 // [s_lo, s_hi) (the last may be partial, finished by the next batch).
 struct GridPlanDev {
+  int n = 0;                       // transform length: grid_transform(p_h)
   double dky = 0;                  // spacing of the ky axis
   double sy = 0;                   // ky(p_h / 2): the shift folded into each atom's phase
   int half = 0;                    // centred antisymmetric axes: S(-k) = conj S(k), columns kx >= 0 only
-  const float2* ay = nullptr;      // [p_h][2]: deconvolution x half-bin phase (parity 0, 1)
+  const float2* ay = nullptr;      // [p_h + 1][2]: deconvolution x half-bin phase (parity 0, 1)
+  const float2* tw = nullptr;      // twiddles of n
   const int4* jobs = nullptr;      // [jobs]: kind (SpeciesSet index), species, first atom, end atom
   const int* job_beg = nullptr;    // [slices + 1] first job of every slice
   const int* atom_beg = nullptr;   // [jobs + 1] atoms of the jobs before
@@ -129,13 +131,13 @@ struct GridWork {
   int* base = nullptr;             // [atoms]: first fine row of every group
   int* order = nullptr;            // [atoms]: the job's atoms sorted by fine row
   int* first = nullptr;            // [atoms + jobs]: first sorted atom of every group, then the atom count
-  int* ptr = nullptr;              // [jobs][2 p_h + 1]: first group of every fine row
+  int* ptr = nullptr;              // [jobs][2 n + 1]: first group of every fine row
   int* groups = nullptr;           // [jobs]
-  unsigned char* used = nullptr;   // [jobs][2 p_h / 16]: a group spreads into this block of fine rows
+  unsigned char* used = nullptr;   // [jobs][2 n / 16]: a group spreads into this block of fine rows
   // one batch
   int ex_cols = 0;                 // columns of E held at a time (a multiple of 128, or pitch)
   float2* ex = nullptr;            // [jobs][kmax][ex_cols]
-  float2* fine = nullptr;          // [jobs][2 p_h][pitch]
+  float2* fine = nullptr;          // [jobs][2 n][pitch]
   float2* s = nullptr;             // [jobs][p_h + 1][pitch]
 };
 struct GridBatch {
@@ -155,9 +157,12 @@ Status launch_tx_gridding(const TxGrid& g, const SpeciesSet& sp, const GridPlanD
                           const std::vector<int>& job_beg, int kmax, long long atoms, const float2* tw_w,
                           const float2* tw_h, void* scratch, size_t scratch_bytes, bool finish, float sig, float2* out,
                           cudaStream_t st, int* launches, bool* finished);
-// Factors of the gridding builder along y for an axis of n points: [r][parity] = the inverse of
-// the spreading kernel's transform times exp(-i pi k parity / n), k = r - n/2.
-std::vector<float2> grid_deconvolution(int n);
+// The smallest edge of the fused transforms that is at least p_h; 0 if there is none.
+int grid_transform(int p_h);
+// Factors of the gridding builder along y for an axis of p_h points and transforms of n: [r][parity] =
+// the inverse of the spreading kernel's transform times exp(-i pi k parity / n), k = r - p_h / 2, r up
+// to and including p_h.
+std::vector<float2> grid_deconvolution(int p_h, int n);
 // Process-wide builder choice for separable grids (TOTEM_TX_*) and gridding scratch bytes.
 int tx_builder_mode();
 // Process-wide: repeated fused slice loops replay as CUDA graphs (totem_set_slice_graphs).
@@ -171,8 +176,8 @@ Status launch_tx_fft_exp(float2* data, int slices, int p_h, int p_w, float sigma
 // Element-wise (-1)^(r+c) and exp for the cuFFT builder.
 Status launch_sign_exp(float2* data, long total, int p_h, int p_w, float sigma_scaled, cudaStream_t st);
 
-// Grid edges of the fused transmission FFT and heights of the gridding builder: powers of two
-// 64..4096 and the mixed-radix edges of TOTEM_MR_WINDOWS.
+// Grid edges of the fused transmission FFT: powers of two 64..4096 and the mixed-radix edges of
+// TOTEM_MR_WINDOWS.
 bool fused_fft_size_ok(int n);
 // Whether the fused transmission FFT takes a p_h x p_w grid of ``slices`` slices: both edges
 // fused_fft_size_ok, the rows of all slices whole row tiles of p_w and the width whole column
@@ -313,7 +318,7 @@ struct WindowOps {
   Status (*tx_rows_inv)(float2* data, long nrows, const float2* tw, cudaStream_t st);
   Status (*tx_cols_exp)(float2* data, int slices, int p_w, const float2* tw, float sig, cudaStream_t st);
   // the gridding builder at height n (grid_cols, grid_cols_inv) and its rows of length n (rows_exp)
-  Status (*grid_cols)(const GridWork& w, int job0, int jobs, const float2* ay, const float2* tw, cudaStream_t st);
+  Status (*grid_cols)(const GridWork& w, int job0, int jobs, int p_h, const float2* ay, const float2* tw, cudaStream_t st);
   Status (*grid_cols_inv)(const TxGrid& g, const SpeciesSet& sp, const GridPlanDev& gp, const GridWork& w, int s_lo,
                           int s_hi, int j_lo, float2* out, const float2* tw, cudaStream_t st);
   Status (*tx_rows_exp)(float2* data, long nrows, const float2* tw, float sig, cudaStream_t st);

@@ -520,8 +520,8 @@ Status totem_session::build_transmission(int path, int* launches) {
     }
     if (gridding) {
       totem::GridPlanDev gp;
-      gp.dky = grid_dky; gp.sy = grid_sy; gp.half = grid_half;
-      gp.ay = grid_ay.as<float2>();
+      gp.n = grid_n; gp.dky = grid_dky; gp.sy = grid_sy; gp.half = grid_half;
+      gp.ay = grid_ay.as<float2>(); gp.tw = tw_grid.as<float2>();
       gp.jobs = grid_jobs.as<int4>(); gp.job_beg = grid_job_beg.as<int>();
       gp.atom_beg = grid_atom_beg.as<int>();
       ran_tx_builder = TOTEM_TX_GRIDDING;
@@ -570,15 +570,16 @@ Status totem_session::build_transmission(int path, int* launches) {
 }
 
 // Uniform separable axes, kx(c) = kx0 + c dkx and ky(r) = ky0 + r dky (the reference's
-// meshgrid of (-P/2 : P/2-1) / (P dx), ToTEM_submit_v1.m:1534-1538), on a grid whose height the
-// fused transforms take admit the gridding builder.  Its job table holds one job per species segment
+// meshgrid of (-P/2 : P/2-1) / (P dx), ToTEM_submit_v1.m:1534-1538), on a grid of up to 4096 rows
+// admit the gridding builder.  Its job table holds one job per species segment
 // of every slice (neutral, ionic, then the correction kinds), in slice order.
 Status totem_session::plan_gridding(const TotemStemArgs* a, const totem::SpeciesHost* const (&kinds)[4]) {
   grid_ok = false;
   grid_job_beg_h.clear();
   grid_atoms = 0;
   grid_kmax = 1;
-  if (!totem::fused_fft_size_ok(p_h) || slices <= 0) return Status::Ok();
+  grid_n = totem::grid_transform(p_h);
+  if (grid_n == 0 || slices <= 0) return Status::Ok();
   auto uniform = [](const double* v, int n, long stride, double* d) {
     *d = (v[(long)(n - 1) * stride] - v[0]) / (n - 1);
     if (!std::isfinite(*d) || *d == 0.0) return false;
@@ -614,7 +615,8 @@ Status totem_session::plan_gridding(const TotemStemArgs* a, const totem::Species
   TOTEM_TRY(upload(grid_jobs, jobs, st));
   TOTEM_TRY(upload(grid_job_beg, grid_job_beg_h, st));
   TOTEM_TRY(upload(grid_atom_beg, atom_beg, st));
-  TOTEM_TRY(upload(grid_ay, totem::grid_deconvolution(p_h), st));
+  TOTEM_TRY(upload(grid_ay, totem::grid_deconvolution(p_h, grid_n), st));
+  TOTEM_TRY(upload(tw_grid, twiddles(grid_n), st));
   grid_ok = true;
   return Status::Ok();
 }
@@ -629,7 +631,7 @@ Status totem_session::plan_gridding(const TotemStemArgs* a, const totem::Species
 // against 2.26 / 2.29 / 2.35 / 2.66 ms.
 bool totem_session::gridding_cheaper() const {
   const double plane = (double)p_h * p_w, jobs = (double)grid_job_beg_h.back();
-  const double per_px = (p_h <= 1024 && is_pow2(p_h)) ? 1e-12 : 4e-12;
+  const double per_px = (grid_n <= 1024 && is_pow2(grid_n)) ? 1e-12 : 4e-12;
   return per_px * jobs * plane + 1.2e-5 < 2.9e-13 * (double)grid_atoms * plane;
 }
 

@@ -204,7 +204,7 @@ struct totem_session {
   int n_rows = 0, n_rows_i = 0, n_corr = 0, n_corr_i = 0, cim_len = 0, ncoef_n = 0, ncoef_i = 0;
 
   // device inputs
-  totem::DevBuf probe, prop, mask_mid, mask_exit, tw_n, tw_pw, tw_ph, gfsf_d;
+  totem::DevBuf probe, prop, mask_mid, mask_exit, tw_n, tw_pw, tw_ph, tw_grid, gfsf_d;
   totem::RowsDev rows_n, rows_i, rows_cn, rows_ci;
   totem::SpeciesRowsDev species_n, species_i;  // the neutral / ionic rows by species (separable grids)
   totem::SpeciesRowsDev species_cn, species_ci;  // the correction rows by species (separable grids)
@@ -213,6 +213,7 @@ struct totem_session {
   // gridding builder (uniform separable axes): job table, deconvolution table, work memory
   bool grid_ok = false;
   double grid_dky = 0, grid_sy = 0;
+  int grid_n = 0;     // transform length of the gridding builder (totem::grid_transform)
   int grid_half = 0;  // centred antisymmetric axes (GridPlanDev::half)
   int grid_kmax = 1;  // atoms of the largest job
   long long grid_atoms = 0;
@@ -266,7 +267,7 @@ struct totem_session {
 
   template <class F>
   void for_each_buf(F&& f) {
-    for (totem::DevBuf* b : {&probe, &prop, &mask_mid, &mask_exit, &tw_n, &tw_pw, &tw_ph, &gfsf_d, &kx_axis, &ky_axis,
+    for (totem::DevBuf* b : {&probe, &prop, &mask_mid, &mask_exit, &tw_n, &tw_pw, &tw_ph, &tw_grid, &gfsf_d, &kx_axis, &ky_axis,
                              &kx, &ky, &s2, &aper_true, &cim, &T, &psi, &part, &acc, &out_result, &out_mid,
                              &ev_slice, &Tb, &hr_wave, &hr_prop, &hr_tf, &hr_w, &hr_work, &hr_exit, &hr_img, &grid_jobs,
                              &grid_job_beg, &grid_atom_beg, &grid_ay, &grid_scratch})

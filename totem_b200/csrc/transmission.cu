@@ -287,7 +287,7 @@ __device__ int block_exclusive_scan(int* cnt, int n, int* warp_sum) {
   return total;
 }
 
-// Fine-grid place of an atom: v in [0, 2 p_h], first row b = ceil(v - GR_W / 2) mod 2 p_h.
+// Fine-grid place of an atom: v in [0, nf], first row b = ceil(v - GR_W / 2) mod nf (nf = 2 n rows).
 __device__ __forceinline__ double fine_row(double y, double dky, int nf) {
   const double t = dky * y;
   return (t - floor(t)) * nf;
@@ -300,10 +300,10 @@ __device__ __forceinline__ int first_row(double v, int nf) {
 // One CTA per job: counting sort of its atoms by first fine row (stable: one warp places 32 atoms
 // at a time in order, so the result does not depend on timing), groups of adjacent atoms with the
 // same y, the first group of every fine row, and the blocks of fine rows a group reaches.
-__global__ void __launch_bounds__(GR_T) k_grid_sort(GridPlanDev gp, SpeciesSet spset, int p_h, GridWork w) {
-  extern __shared__ int cnt[];  // [2 p_h + 1]
+__global__ void __launch_bounds__(GR_T) k_grid_sort(GridPlanDev gp, SpeciesSet spset, GridWork w) {
+  extern __shared__ int cnt[];  // [2 n + 1]
   __shared__ int warp_sum[GR_T / 32];
-  const int nf = 2 * p_h, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int nf = 2 * gp.n, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int4 jb = gp.jobs[blockIdx.x];
   const int K = jb.w - jb.z;
   const double* pos = spset.k[jb.x & 3].pos + 2L * jb.z;
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(128) k_grid_phases(GridPlanDev gp, SpeciesSet 
     if (h < 128) {  // thread (q, k): weight k of group q
       const int q = q0 + threadIdx.x / GR_W, k = threadIdx.x % GR_W;
       if (q < groups) {
-        const double v = fine_row(pos[2L * order[first[q]] + 1], gp.dky, 2 * g.p_h);
+        const double v = fine_row(pos[2L * order[first[q]] + 1], gp.dky, 2 * gp.n);
         const double d = (ceil(v - GR_W / 2) + k - v) / (GR_W / 2);
         wgt[GR_W * q + k] = (float)(bessel_i0(GR_BETA * sqrt(fmax(1.0 - d * d, 0.0))) * (1.0 / bessel_i0(GR_BETA)));
       }
@@ -437,8 +437,8 @@ __device__ __forceinline__ void spread_at(float2 (&acc)[GR_ROWS], const float* w
 // reach the block in sorted order.  All lanes take the same group, so its offset picks one of the 23
 // unrolled bodies without divergence and the weights are uniform loads; E is loaded four groups
 // ahead of its use.
-__global__ void __launch_bounds__(128) k_grid_spread(GridPlanDev gp, int p_h, int job0, int col0, GridWork w) {
-  const int nf = 2 * p_h, f0 = blockIdx.y * GR_ROWS, job = job0 + blockIdx.z;
+__global__ void __launch_bounds__(128) k_grid_spread(GridPlanDev gp, int job0, int col0, GridWork w) {
+  const int nf = 2 * gp.n, f0 = blockIdx.y * GR_ROWS, job = job0 + blockIdx.z;
   const int h = col0 + blockIdx.x * 128 + threadIdx.x;
   if (!w.used[(long)job * (nf / GR_ROWS) + blockIdx.y]) return;
   const int hc = min(h, w.pitch - 1);
@@ -513,6 +513,7 @@ __global__ void __launch_bounds__(256) k_grid_combine(TxGrid g, SpeciesSet spset
 // Where the parts of the work memory lie (base may be null: sizes only); returns its bytes.
 // ``batch`` jobs in a batch.
 size_t grid_work(int p_h, int p_w, int half, int kmax, int jobs, long long atoms, int batch, char* base, GridWork* w) {
+  const size_t n = grid_transform(p_h);
   w->kmax = kmax;
   w->half = half;
   w->cols = half ? p_w / 2 + 1 : p_w;
@@ -529,14 +530,14 @@ size_t grid_work(int p_h, int p_w, int half, int kmax, int jobs, long long atoms
   w->base = reinterpret_cast<int*>(take(na * sizeof(int)));
   w->order = reinterpret_cast<int*>(take(na * sizeof(int)));
   w->first = reinterpret_cast<int*>(take((na + nj) * sizeof(int)));
-  w->ptr = reinterpret_cast<int*>(take(nj * (2 * (size_t)p_h + 1) * sizeof(int)));
+  w->ptr = reinterpret_cast<int*>(take(nj * (2 * n + 1) * sizeof(int)));
   w->groups = reinterpret_cast<int*>(take(nj * sizeof(int)));
-  w->used = reinterpret_cast<unsigned char*>(take(nj * (2 * (size_t)p_h / GR_ROWS)));
+  w->used = reinterpret_cast<unsigned char*>(take(nj * (2 * n / GR_ROWS)));
   // E is at most as large as two fine columns' worth of rows; jobs of more atoms take it in pieces
   const long room = 4L * p_h * w->pitch / kmax / 128 * 128;
   w->ex_cols = room >= w->pitch ? w->pitch : (int)std::max(room, 128L);
   w->ex = reinterpret_cast<float2*>(take(nb * kmax * w->ex_cols * sizeof(float2)));
-  w->fine = reinterpret_cast<float2*>(take(nb * 2 * p_h * row));
+  w->fine = reinterpret_cast<float2*>(take(nb * 2 * n * row));
   w->s = reinterpret_cast<float2*>(take(nb * (p_h + 1) * row));
   return off;
 }
@@ -612,12 +613,21 @@ Status launch_tx_species(const TxGrid& g, const SpeciesSet& sp, float2* out, cud
   return cuda_status(cudaGetLastError(), "k_tx_species");
 }
 
-std::vector<float2> grid_deconvolution(int n) {
+int grid_transform(int p_h) {
+  if (p_h < 1 || p_h > 4096) return 0;
+  int n = 64;  // the powers of two, then a mixed-radix edge below the one found
+  while (n < p_h) n *= 2;
+  for (int m = p_h; m < n; ++m)
+    if (radix_window_ops(m)) return m;
+  return n;
+}
+
+std::vector<float2> grid_deconvolution(int p_h, int n) {
   // transform of the spreading kernel at xi = k / (2 n): W sinh(z) / (z I0(beta))
   const double pi = 3.14159265358979323846, i0 = bessel_i0(GR_BETA);
-  std::vector<float2> t(2 * (size_t)n);
-  for (int r = 0; r < n; ++r) {
-    const double k = r - n / 2, a = pi * GR_W * k / (2.0 * n);
+  std::vector<float2> t(2 * ((size_t)p_h + 1));
+  for (int r = 0; r <= p_h; ++r) {
+    const double k = r - p_h / 2, a = pi * GR_W * k / (2.0 * n);
     const double z = std::sqrt(GR_BETA * GR_BETA - a * a);
     const double d = z * i0 / (GR_W * std::sinh(z));
     t[2 * r] = make_float2((float)d, 0.f);
@@ -693,9 +703,9 @@ Status launch_tx_gridding(const TxGrid& g, const SpeciesSet& sp, const GridPlanD
     batches = grid_batches(job_beg, per_batch);
   }
   if (jobs > 0) {
-    const size_t smem = sizeof(int) * (2 * (size_t)g.p_h + 1);
+    const size_t smem = sizeof(int) * (2 * (size_t)gp.n + 1);
     TOTEM_TRY(ensure_smem((const void*)k_grid_sort, smem));
-    k_grid_sort<<<jobs, GR_T, smem, st>>>(gp, sp, g.p_h, w);
+    k_grid_sort<<<jobs, GR_T, smem, st>>>(gp, sp, w);
     TOTEM_TRY(cuda_status(cudaGetLastError(), "k_grid_sort"));
     ++*launches;
   }
@@ -707,11 +717,11 @@ Status launch_tx_gridding(const TxGrid& g, const SpeciesSet& sp, const GridPlanD
         k_grid_phases<<<dim3(cx, (unsigned)std::min((kmax + 15) / 16, 1024), nj), 128, 0, st>>>(gp, sp, g, b.j_lo,
                                                                                                col0, w);
         TOTEM_TRY(cuda_status(cudaGetLastError(), "k_grid_phases"));
-        k_grid_spread<<<dim3(cx, 2 * g.p_h / GR_ROWS, nj), 128, 0, st>>>(gp, g.p_h, b.j_lo, col0, w);
+        k_grid_spread<<<dim3(cx, 2 * gp.n / GR_ROWS, nj), 128, 0, st>>>(gp, b.j_lo, col0, w);
         TOTEM_TRY(cuda_status(cudaGetLastError(), "k_grid_spread"));
         *launches += 2;
       }
-      TOTEM_TRY(TOTEM_GRID_DISPATCH(g.p_h, grid_cols, grid_cols, w, b.j_lo, nj, gp.ay, tw_h, st));
+      TOTEM_TRY(TOTEM_GRID_DISPATCH(gp.n, grid_cols, grid_cols, w, b.j_lo, nj, g.p_h, gp.ay, gp.tw, st));
       ++*launches;
     }
     if (finish) {

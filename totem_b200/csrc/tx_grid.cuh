@@ -5,15 +5,18 @@
 // Per job (one species of one slice) the builder needs, on a separable grid with a uniform ky axis
 // (ky(r) = ky(P/2) + (r - P/2) dky, P = p_h),
 //   S(r, c) = sum_a exp(-2 pi i kx(c) x_a) exp(-2 pi i ky(r) y_a).
-// The x factor is evaluated directly; the y factor is a type-1 non-uniform FFT per column:
-//   k_grid_sort    sorts the job's atoms by their place on a fine y grid of 2P rows and joins atoms
+// The x factor is evaluated directly; the y factor is a type-1 non-uniform FFT per column, with N the
+// smallest edge of the fused transforms that is at least P (GridPlanDev::n; N = P where the height is
+// such an edge, and the inverse transform is fused too):
+//   k_grid_sort    sorts the job's atoms by their place on a fine y grid of 2N rows and joins atoms
 //                  of equal y into one group;
 //   k_grid_phases  E[group][c] = sum over the group's atoms of exp(-2 pi i kx(c) x_a), and the
 //                  group's GR_W spreading weights;
 //   k_grid_spread  the fine rows: sum over groups of weight times E, sixteen rows of a column in
 //                  one thread's registers, the lanes of a warp along c;
-//   k_grid_cols    per column tile: the fine column's transform (two P-point FFTs, fine rows of
-//                  even and odd index) divided by the spreading kernel's transform: S;
+//   k_grid_cols    per column tile: the fine column's transform (two N-point FFTs, fine rows of
+//                  even and odd index), its P central frequencies divided by the spreading kernel's
+//                  transform: S;
 //   k_grid_cols_inv  form factors, the sum over the slice's jobs, and the inverse column FFT;
 //   k_rows_exp       the inverse row FFT and T = exp(i sigma V).
 // (k_grid_combine in transmission.cu writes the sum itself instead, where per-atom correction rows
@@ -122,7 +125,7 @@ using GridTile = ColCfg<N, 4, (N >= 2048) ? 4 : 0>;
 // (the same thread writes and reads back its elements).
 template <int N>
 __global__ void __launch_bounds__(GridTile<N>::G * GridTile<N>::T, GridTile<N>::MINB)
-    k_grid_cols(GridWork w, int job0, const float4* __restrict__ ay, int tiles, const float2* __restrict__ tw) {
+    k_grid_cols(GridWork w, int job0, int p_h, const float4* __restrict__ ay, int tiles, const float2* __restrict__ tw) {
   constexpr int P = GridTile<N>::P, T = GridTile<N>::T, G = GridTile<N>::G;
   extern __shared__ float2 sh[];
   float2* s_tw = sh;
@@ -131,7 +134,7 @@ __global__ void __launch_bounds__(GridTile<N>::G * GridTile<N>::T, GridTile<N>::
   const int j = threadIdx.x / G, g = threadIdx.x - j * G;
   const float2* __restrict__ fine = w.fine + (long)job * 2 * N * w.pitch + col0 + g;
   const unsigned char* __restrict__ used = w.used + (long)(job0 + job) * (2 * N / GR_ROWS);
-  float2* S = w.s + (long)job * (N + 1) * w.pitch + col0 + g;
+  float2* S = w.s + (long)job * (p_h + 1) * w.pitch + col0 + g;
   load_twiddles<N>(s_tw, tw);
   static_for<0, 2>([&](auto parity) {
     constexpr int e = decltype(parity)::value;
@@ -146,16 +149,20 @@ __global__ void __launch_bounds__(GridTile<N>::G * GridTile<N>::T, GridTile<N>::
 #pragma unroll
     for (int m = 0; m < P; ++m) {
       if (m % 8 == 0) asm volatile("" ::: "memory");  // eight loads of S in flight: all of them would spill
-      const int k = j + m * T, r = m < P / 2 ? k + N / 2 : k - N / 2;  // ky = r - N / 2
-      const float4 a = __ldg(ay + r);
-      float2* dst = S + r * w.pitch;
-      if (e == 0) {
-        *dst = cscale(v[m], a.x);
-      } else {
-        const float2 odd = cmul(v[m], make_float2(a.z, a.w)), even = *dst;
-        *dst = cadd(even, odd);
-        // row N, ky = +N / 2, which the conjugate half of row 0 (ky = -N / 2) needs
-        if (m == P / 2 && j == 0) S[N * w.pitch] = csub(even, odd);
+      // frequency ky = k or k - N is row r = ky + p_h / 2; one row more, ky = +p_h / 2, is what the
+      // conjugate half of row 0 (ky = -p_h / 2) needs.  With p_h = N that is row 0's own frequency
+      // with the odd half's phase turned by pi.
+      const int k = j + m * T, r = (m < P / 2 ? k : k - N) + p_h / 2;
+      if (r >= 0 && r <= p_h) {
+        const float4 a = __ldg(ay + r);
+        float2* dst = S + r * w.pitch;
+        if (e == 0) {
+          *dst = cscale(v[m], a.x);
+        } else {
+          const float2 odd = cmul(v[m], make_float2(a.z, a.w)), even = *dst;
+          *dst = cadd(even, odd);
+          if (r == 0 && p_h == N) S[N * w.pitch] = csub(even, odd);
+        }
       }
     }
   });
@@ -308,14 +315,14 @@ __global__ void __launch_bounds__(RowCfg<N>::G * RowCfg<N>::T, RowCfg<N>::MINB)
 }
 
 template <int N>
-Status grid_cols(const GridWork& w, int job0, int jobs, const float2* ay, const float2* tw, cudaStream_t st) {
+Status grid_cols(const GridWork& w, int job0, int jobs, int p_h, const float2* ay, const float2* tw, cudaStream_t st) {
   constexpr int T = GridTile<N>::T, G = GridTile<N>::G;
   static_assert(2 * N % GR_ROWS == 0, "whole blocks of fine rows");
   const size_t smem = sizeof(float2) * (Fft<N>::tw_size + ColLayout<N, G>::size(G));
   TOTEM_TRY(ensure_smem((const void*)k_grid_cols<N>, smem));
   if (w.pitch % G) return Status::Err(TOTEM_ERR_STATE, "gridding pitch not a multiple of the column tile");
   const int tiles = (w.cols + G - 1) / G;
-  k_grid_cols<N><<<(unsigned)((long)jobs * tiles), G * T, smem, st>>>(w, job0, reinterpret_cast<const float4*>(ay),
+  k_grid_cols<N><<<(unsigned)((long)jobs * tiles), G * T, smem, st>>>(w, job0, p_h, reinterpret_cast<const float4*>(ay),
                                                                         tiles, tw);
   return cuda_status(cudaGetLastError(), "k_grid_cols");
 }
