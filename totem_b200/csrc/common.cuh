@@ -342,10 +342,10 @@ Status launch_combine(const double* acc, const double* gfsf, int w_num, long ad,
 // ---------------------------------------------------------------------------------------------
 // Plain path (cuFFT + element-wise kernels)
 // ---------------------------------------------------------------------------------------------
-Status launch_plain_init(float2* psi, const float2* probe, int h, int w, int items, int item0, int depth,
-                         cudaStream_t st);
-Status launch_plain_gather_mul(float2* psi, const float2* tslice, int h, int w, int items, int item0,
-                               ScanGeom geo, cudaStream_t st);
+// psi = (psi * scale) .* T window (tslice null: T = 1), or with ``probe`` the item's probe instead of
+// psi on the right.
+Status launch_plain_gather_mul(float2* psi, const float2* probe, const float2* tslice, int h, int w, int items,
+                               int item0, ScanGeom geo, float scale, cudaStream_t st);
 Status launch_plain_mul(float2* psi, const float2* m, int vol, int items, cudaStream_t st);
 Status launch_plain_scale(float2* psi, float s, long total, cudaStream_t st);
 // HRTEM on cuFFT: work[k] = spec .* tf[k] for k < planes (vol elements each), and

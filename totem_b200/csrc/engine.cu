@@ -815,10 +815,10 @@ Status totem_session::slice_loop(int path, int batch, bool batch_fixed, int col_
         cufftHandle p;
         TOTEM_TRY(plan(h, w, items, &p));
         float2* ps = psi.as<float2>();
-        TOTEM_TRY(totem::launch_plain_init(ps, probe.as<float2>(), h, w, items, (int)item0, depth, stream));
-        ++*launches;
         for (int k = 0; k < slices; ++k) {
-          TOTEM_TRY(totem::launch_plain_gather_mul(ps, Tp + (size_t)k * plane, h, w, items, (int)item0, geo, stream));
+          // the probe enters with the first slice's T, the last IFFT's 1 / N^2 with each later one's
+          TOTEM_TRY(totem::launch_plain_gather_mul(ps, k == 0 ? probe.as<float2>() : nullptr, Tp + (size_t)k * plane, h,
+                                                   w, items, (int)item0, geo, k == 0 ? 1.f : 1.f / (float)vol, stream));
           TOTEM_CUFFT(cufftExecC2C(p, (cufftComplex*)ps, (cufftComplex*)ps, CUFFT_FORWARD));
           TOTEM_TRY(totem::launch_plain_mul(ps, prop.as<float2>(), (int)vol, items, stream));
           *launches += 3;
@@ -828,14 +828,21 @@ Status totem_session::slice_loop(int path, int batch, bool batch_fixed, int col_
                                                  part_e + ev_mid * part_stride, nblk, stream));
             ++*launches;
           }
-          TOTEM_CUFFT(cufftExecC2C(p, (cufftComplex*)ps, (cufftComplex*)ps, CUFFT_INVERSE));
-          TOTEM_TRY(totem::launch_plain_scale(ps, 1.f / (float)vol, (long)items * vol, stream));
+          // the exit detectors' FFT cancels the last slice's IFFT: they take its spectrum
+          if (k < slices - 1) {
+            TOTEM_CUFFT(cufftExecC2C(p, (cufftComplex*)ps, (cufftComplex*)ps, CUFFT_INVERSE));
+            ++*launches;
+          }
+        }
+        if (slices == 0) {  // no specimen: the probes' own spectra
+          TOTEM_TRY(totem::launch_plain_gather_mul(ps, probe.as<float2>(), nullptr, h, w, items, (int)item0, geo, 1.f,
+                                                   stream));
+          TOTEM_CUFFT(cufftExecC2C(p, (cufftComplex*)ps, (cufftComplex*)ps, CUFFT_FORWARD));
           *launches += 2;
         }
-        TOTEM_CUFFT(cufftExecC2C(p, (cufftComplex*)ps, (cufftComplex*)ps, CUFFT_FORWARD));
         TOTEM_TRY(totem::launch_plain_detect(ps, mask_exit.as<float>(), aper_num, (int)vol, items,
                                              part_e + exit_event * part_stride, nblk, stream));
-        *launches += 2;
+        ++*launches;
       }
       for (int e = 0; e < n_events; ++e) {
         TOTEM_TRY(totem::launch_det_reduce(part_e + e * part_stride, nblk, aper_num, items, (int)item0, depth,
@@ -1079,15 +1086,12 @@ Status totem_session::hrtem_plain(const TotemHrtemArgs* hr, TotemHrtemOut* out, 
   cufftHandle one;
   TOTEM_TRY(plan(n, n, 1, &one));
   float2* ps = psi.as<float2>();
-  TOTEM_CUDA(cudaMemcpyAsync(ps, hr_wave.p, vol * sizeof(float2), cudaMemcpyDeviceToDevice, stream));
   for (int k = 0; k < slices; ++k) {
-    TOTEM_TRY(totem::launch_plain_gather_mul(ps, Tp + (size_t)k * vol, n, n, 1, 0, geo, stream));
+    TOTEM_TRY(totem::launch_plain_gather_mul(ps, k == 0 ? hr_wave.as<float2>() : nullptr, Tp + (size_t)k * vol, n, n, 1,
+                                             0, geo, k == 0 ? 1.f : 1.f / (float)vol, stream));
     TOTEM_CUFFT(cufftExecC2C(one, (cufftComplex*)ps, (cufftComplex*)ps, CUFFT_FORWARD));
     TOTEM_TRY(totem::launch_plain_mul(ps, hr_prop.as<float2>(), (int)vol, 1, stream));
-    if (k < slices - 1) {
-      TOTEM_CUFFT(cufftExecC2C(one, (cufftComplex*)ps, (cufftComplex*)ps, CUFFT_INVERSE));
-      TOTEM_TRY(totem::launch_plain_scale(ps, 1.f / (float)vol, (long)vol, stream));
-    }
+    if (k < slices - 1) TOTEM_CUFFT(cufftExecC2C(one, (cufftComplex*)ps, (cufftComplex*)ps, CUFFT_INVERSE));
   }
   const float scale = 1.f / ((float)n * (float)n);
   const bool want_exit = out && (out->exit_re || out->exit_im);
@@ -1162,15 +1166,12 @@ Status totem_session::cbed(double* pattern) {
   } else {
     cufftHandle p;
     TOTEM_TRY(plan(h, w, w_num, &p));
-    TOTEM_TRY(totem::launch_plain_init(ps, probe.as<float2>(), h, w, w_num, 0, depth, stream));
     for (int k = 0; k < slices; ++k) {
-      TOTEM_TRY(totem::launch_plain_gather_mul(ps, Tp + (size_t)k * plane, h, w, w_num, 0, geo, stream));
+      TOTEM_TRY(totem::launch_plain_gather_mul(ps, k == 0 ? probe.as<float2>() : nullptr, Tp + (size_t)k * plane, h, w,
+                                               w_num, 0, geo, k == 0 ? 1.f : 1.f / (float)vol, stream));
       TOTEM_CUFFT(cufftExecC2C(p, (cufftComplex*)ps, (cufftComplex*)ps, CUFFT_FORWARD));
       TOTEM_TRY(totem::launch_plain_mul(ps, prop.as<float2>(), (int)vol, w_num, stream));
-      if (k < slices - 1) {
-        TOTEM_CUFFT(cufftExecC2C(p, (cufftComplex*)ps, (cufftComplex*)ps, CUFFT_INVERSE));
-        TOTEM_TRY(totem::launch_plain_scale(ps, 1.f / (float)vol, (long)w_num * vol, stream));
-      }
+      if (k < slices - 1) TOTEM_CUFFT(cufftExecC2C(p, (cufftComplex*)ps, (cufftComplex*)ps, CUFFT_INVERSE));
     }
   }
   TOTEM_TRY(cbed_out.ensure(vol * sizeof(double)));

@@ -1,46 +1,51 @@
-// Plain slice loop: cuFFT batched transforms plus one element-wise kernel per step.
+// Plain slice loop: cuFFT batched transforms plus one element-wise kernel between each two.
 //
-// This is the comparator the fused path is timed against; its steps mirror the reference's
-// sequence (cuda_source_lobato.cu:1304-1458): initKernel_W, w_p_pointMul, FFT, w_constM_pointMul,
-// [mid detectors], IFFT, scaler, ..., final FFT, detectors.  Plans are cached by the engine and
-// nothing synchronises between launches.  The same kernels (plus the transfer-function multiply
-// and the image sum below) carry HRTEM on grids the fused passes do not take.
+// This is the comparator the fused path is timed against, and what windows outside the fused sizes
+// run on.  Its steps follow the reference's sequence (cuda_source_lobato.cu:1304-1458): initKernel_W,
+// w_p_pointMul, FFT, w_constM_pointMul, [mid detectors], IFFT, scaler, ..., detectors, with the
+// probe's copy and the 1 / N^2 taken into the multiply by T (the same roundings), and without the
+// last IFFT, scaler and FFT, which cancel.  Plans are cached by the engine and nothing synchronises
+// between launches.  The same kernels (plus the transfer-function multiply and the image sum below)
+// carry HRTEM on grids the fused passes do not take.
+//
+// The element-wise kernels are bound by memory: a grid row of blocks per item keeps the index
+// arithmetic to one 32-bit division (64-bit divisions per element made each of them two to three
+// times as long as its traffic takes).
 #include "common.cuh"
 
 namespace totem {
 
 namespace {
 
-__global__ void k_plain_init(float2* __restrict__ psi, const float2* __restrict__ probe, int vol, int items,
-                             int item0, int depth) {
-  const long total = (long)items * vol;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const int item = (int)(i / vol), e = (int)(i % vol);
-    const int w = (item0 + item) / depth;
-    psi[i] = probe[(long)w * vol + e];
+// psi = (src * scale) * T[window]; src is the item's wave, or its probe when ``probe`` is given.  T is 1
+// where ``tslice`` is null.
+__global__ void __launch_bounds__(256) k_plain_gather_mul(float2* __restrict__ psi, const float2* __restrict__ probe,
+                                                          const float2* __restrict__ tslice, int h, int w, int items,
+                                                          int item0, ScanGeom geo, float scale) {
+  const int vol = h * w;
+  for (int item = blockIdx.y; item < items; item += gridDim.y) {
+    const int gi = item0 + item, pos = gi % geo.depth;
+    const float2* t0 = tslice + (long)(geo.begin_row + (pos / geo.width_red) * geo.step) * geo.p_width +
+                       geo.begin_col + (pos % geo.width_red) * geo.step;
+    float2* dst = psi + (long)item * vol;
+    const float2* src = probe != nullptr ? probe + (long)(gi / geo.depth) * vol : dst;
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < vol; e += gridDim.x * blockDim.x) {
+      const int r = e / w, c = e - r * w;
+      const float2 t = tslice != nullptr ? __ldg(t0 + (long)r * geo.p_width + c) : make_float2(1.f, 0.f);
+      const float2 u = src[e], v = make_float2(u.x * scale, u.y * scale);
+      dst[e] = make_float2(v.x * t.x - v.y * t.y, v.x * t.y + v.y * t.x);
+    }
   }
 }
 
-__global__ void k_plain_gather_mul(float2* __restrict__ psi, const float2* __restrict__ tslice, int h, int w,
-                                   int items, int item0, ScanGeom geo) {
-  const long vol = (long)h * w, total = items * vol;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const int item = (int)(i / vol);
-    const int e = (int)(i % vol), r = e / w, c = e % w;
-    const int pos = (item0 + item) % geo.depth;
-    const int x0 = geo.begin_row + (pos / geo.width_red) * geo.step;
-    const int y0 = geo.begin_col + (pos % geo.width_red) * geo.step;
-    const float2 t = tslice[(long)(x0 + r) * geo.p_width + y0 + c];
-    const float2 v = psi[i];
-    psi[i] = make_float2(v.x * t.x - v.y * t.y, v.x * t.y + v.y * t.x);
-  }
-}
-
-__global__ void k_plain_mul(float2* __restrict__ psi, const float2* __restrict__ m, int vol, long total) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-    const float2 t = m[i % vol];
-    const float2 v = psi[i];
-    psi[i] = make_float2(v.x * t.x - v.y * t.y, v.x * t.y + v.y * t.x);
+__global__ void __launch_bounds__(256) k_plain_mul(float2* __restrict__ psi, const float2* __restrict__ m, int vol,
+                                                   int items) {
+  for (int item = blockIdx.y; item < items; item += gridDim.y) {
+    float2* p = psi + (long)item * vol;
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < vol; e += gridDim.x * blockDim.x) {
+      const float2 t = __ldg(m + e), v = p[e];
+      p[e] = make_float2(v.x * t.x - v.y * t.y, v.x * t.y + v.y * t.x);
+    }
   }
 }
 
@@ -125,23 +130,21 @@ inline int grid_for(long total) { return (int)std::min<long>((total + 255) / 256
 
 }  // namespace
 
-Status launch_plain_init(float2* psi, const float2* probe, int h, int w, int items, int item0, int depth,
-                         cudaStream_t st) {
-  const long total = (long)items * h * w;
-  k_plain_init<<<grid_for(total), 256, 0, st>>>(psi, probe, h * w, items, item0, depth);
-  return cuda_status(cudaGetLastError(), "k_plain_init");
+// blocks of 256 threads along an item of vol elements (four elements each), items along y
+inline dim3 item_grid(int vol, int items) {
+  return dim3((unsigned)std::max(1, (vol + 1023) / 1024), (unsigned)std::min(items, 65535));
 }
 
-Status launch_plain_gather_mul(float2* psi, const float2* tslice, int h, int w, int items, int item0, ScanGeom geo,
-                               cudaStream_t st) {
-  const long total = (long)items * h * w;
-  k_plain_gather_mul<<<grid_for(total), 256, 0, st>>>(psi, tslice, h, w, items, item0, geo);
+Status launch_plain_gather_mul(float2* psi, const float2* probe, const float2* tslice, int h, int w, int items,
+                               int item0, ScanGeom geo, float scale, cudaStream_t st) {
+  if (items <= 0) return Status::Ok();
+  k_plain_gather_mul<<<item_grid(h * w, items), 256, 0, st>>>(psi, probe, tslice, h, w, items, item0, geo, scale);
   return cuda_status(cudaGetLastError(), "k_plain_gather_mul");
 }
 
 Status launch_plain_mul(float2* psi, const float2* m, int vol, int items, cudaStream_t st) {
-  const long total = (long)items * vol;
-  k_plain_mul<<<grid_for(total), 256, 0, st>>>(psi, m, vol, total);
+  if (items <= 0) return Status::Ok();
+  k_plain_mul<<<item_grid(vol, items), 256, 0, st>>>(psi, m, vol, items);
   return cuda_status(cudaGetLastError(), "k_plain_mul");
 }
 
