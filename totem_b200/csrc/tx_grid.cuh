@@ -123,10 +123,12 @@ using GridTile = ColCfg<N, 4, (N >= 2048) ? 4 : 0>;
 
 // S of the jobs of a batch from their fine rows.  The even and odd spectra are added through S itself
 // (the same thread writes and reads back its elements).
-template <int N>
+// WHOLE: the grid has N rows (known at compile time, so that no row is tested).
+template <int N, bool WHOLE>
 __global__ void __launch_bounds__(GridTile<N>::G * GridTile<N>::T, GridTile<N>::MINB)
-    k_grid_cols(GridWork w, int job0, int p_h, const float4* __restrict__ ay, int tiles, const float2* __restrict__ tw) {
+    k_grid_cols(GridWork w, int job0, int rows, const float4* __restrict__ ay, int tiles, const float2* __restrict__ tw) {
   constexpr int P = GridTile<N>::P, T = GridTile<N>::T, G = GridTile<N>::G;
+  const int p_h = WHOLE ? N : rows;
   extern __shared__ float2 sh[];
   float2* s_tw = sh;
   float2* s_x = sh + Fft<N>::tw_size;
@@ -153,7 +155,7 @@ __global__ void __launch_bounds__(GridTile<N>::G * GridTile<N>::T, GridTile<N>::
       // conjugate half of row 0 (ky = -p_h / 2) needs.  With p_h = N that is row 0's own frequency
       // with the odd half's phase turned by pi.
       const int k = j + m * T, r = (m < P / 2 ? k : k - N) + p_h / 2;
-      if (r >= 0 && r <= p_h) {
+      if (WHOLE || (r >= 0 && r <= p_h)) {
         const float4 a = __ldg(ay + r);
         float2* dst = S + r * w.pitch;
         if (e == 0) {
@@ -161,7 +163,7 @@ __global__ void __launch_bounds__(GridTile<N>::G * GridTile<N>::T, GridTile<N>::
         } else {
           const float2 odd = cmul(v[m], make_float2(a.z, a.w)), even = *dst;
           *dst = cadd(even, odd);
-          if (r == 0 && p_h == N) S[N * w.pitch] = csub(even, odd);
+          if (WHOLE && m == P / 2 && j == 0) S[N * w.pitch] = csub(even, odd);
         }
       }
     }
@@ -319,11 +321,11 @@ Status grid_cols(const GridWork& w, int job0, int jobs, int p_h, const float2* a
   constexpr int T = GridTile<N>::T, G = GridTile<N>::G;
   static_assert(2 * N % GR_ROWS == 0, "whole blocks of fine rows");
   const size_t smem = sizeof(float2) * (Fft<N>::tw_size + ColLayout<N, G>::size(G));
-  TOTEM_TRY(ensure_smem((const void*)k_grid_cols<N>, smem));
+  const auto kernel = p_h == N ? k_grid_cols<N, true> : k_grid_cols<N, false>;
+  TOTEM_TRY(ensure_smem((const void*)kernel, smem));
   if (w.pitch % G) return Status::Err(TOTEM_ERR_STATE, "gridding pitch not a multiple of the column tile");
   const int tiles = (w.cols + G - 1) / G;
-  k_grid_cols<N><<<(unsigned)((long)jobs * tiles), G * T, smem, st>>>(w, job0, p_h, reinterpret_cast<const float4*>(ay),
-                                                                        tiles, tw);
+  kernel<<<(unsigned)((long)jobs * tiles), G * T, smem, st>>>(w, job0, p_h, reinterpret_cast<const float4*>(ay), tiles, tw);
   return cuda_status(cudaGetLastError(), "k_grid_cols");
 }
 
