@@ -31,6 +31,24 @@ Status ensure_smem(const void* func, size_t bytes);
 // Set the calling thread's message returned by totem_last_error().
 void set_last_error(const std::string& msg);
 
+// Launches kernel<<<grid, block, smem, st>>>(args...); with ``overlap`` as a programmatic dependent launch
+// (the kernel waits for its predecessor itself, wait_for_previous_kernel in fft.cuh).
+template <class... Params, class... Args>
+cudaError_t launch_kernel(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
+                          bool overlap, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 #define TOTEM_CUDA(call)                                              \
   do {                                                                \
     cudaError_t _e = (call);                                          \
@@ -241,6 +259,7 @@ struct SliceLoopArgs {
   int skip_band = 0;               // 1: the passes leave out band_columns(n) (band_skip_ok)
   int skip_rows = 0;               // 1: the propagator is zero on the rows BandRows<n> (band_rows_ok)
   int row_variant = 0;             // row-pass variant (multislice.cu, row_pass)
+  int overlap = 0;                 // 1: the pass may be launched before the one ahead of it has ended
 };
 // Number of column tiles per item (detector partial sums per probe) of a column-pass variant.
 int col_blocks(int n, int variant = 0);

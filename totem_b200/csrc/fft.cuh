@@ -662,6 +662,12 @@ __device__ __forceinline__ auto group_sync(int g) {
   else return SyncBlock{};
 }
 
+// Programmatic dependent launch: a kernel launched with the attribute may start while the one before
+// it in the stream still runs, and waits here for that one's results; the other call lets the next
+// kernel start.  Both do nothing in a kernel launched without the attribute.
+__device__ __forceinline__ void wait_for_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Cooperative copy of the twiddle tables into shared memory (caller synchronises afterwards).
 template <int N>
 __device__ __forceinline__ void load_twiddles(float2* dst, const float2* __restrict__ src) {

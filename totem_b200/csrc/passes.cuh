@@ -34,8 +34,9 @@ Status row_pass_launch(const SliceLoopArgs& a, const void* tslice, cudaStream_t 
   TOTEM_TRY(ensure_smem((const void*)k_row_pass<N, FIRST, TB16, CTAS, SKIP>, smem));
   const long rows = (long)a.items * N;
   const float scale = FIRST ? 1.f : 1.f / ((float)N * (float)N);
-  k_row_pass<N, FIRST, TB16, CTAS, SKIP><<<(unsigned)(rows / G), G * T, smem, st>>>(a, tslice, scale);
-  return cuda_status(cudaGetLastError(), "k_row_pass");
+  return cuda_status(launch_kernel(k_row_pass<N, FIRST, TB16, CTAS, SKIP>, (unsigned)(rows / G), G * T, smem, st,
+                                   a.overlap != 0, a, tslice, scale),
+                     "k_row_pass");
 }
 
 // the zero-band skip (a.skip_band) chosen at launch; windows without a band skip nothing
@@ -92,9 +93,10 @@ Status col_pass_launch(const SliceLoopArgs& a, int flags, TileSkip skip, cudaStr
   constexpr int G = ColCfg<N, CTAS128, GW>::G, T = ColCfg<N>::T;
   const size_t smem = sizeof(float2) * (Fft<N>::tw_size + ColLayout<N, G>::size(G));
   TOTEM_TRY(ensure_smem((const void*)k_col_pass<N, PREFETCH, CTAS128, GW, ROWS>, smem));
-  k_col_pass<N, PREFETCH, CTAS128, GW, ROWS>
-      <<<(unsigned)((long)a.items * (N / G - skip.nskip)), G * T, smem, st>>>(a, flags, skip);
-  return cuda_status(cudaGetLastError(), "k_col_pass");
+  return cuda_status(launch_kernel(k_col_pass<N, PREFETCH, CTAS128, GW, ROWS>,
+                                   (unsigned)((long)a.items * (N / G - skip.nskip)), G * T, smem, st, a.overlap != 0, a,
+                                   flags, skip),
+                     "k_col_pass");
 }
 
 // the zero rows (a.skip_rows) chosen at launch; windows without a band of rows skip nothing

@@ -338,6 +338,7 @@ struct totem_session {
   Status transmission_for(int t_storage, const void** t, size_t* slice_bytes, int* launches);
   Status run_graphed(const std::vector<long long>& key, const std::function<Status()>& enqueue, int* launches);
   void drop_graph();
+  Status spectrum_loop(totem::SliceLoopArgs s, const char* t, size_t tslice_bytes, int* launches);
   Status hrtem(const TotemHrtemArgs* h, TotemHrtemOut* out);
   Status hrtem_plain(const TotemHrtemArgs* hr, TotemHrtemOut* out, const float2* Tp);
   Status cbed(double* pattern);

@@ -51,7 +51,9 @@ __device__ __forceinline__ void row_tile(float2* __restrict__ psi_item, const vo
   float2* s_x = sh + Fft<N>::tw_size;
   const int g = threadIdx.x / T, j = threadIdx.x - g * T;
   const int row = row0 + g;
+  let_next_kernel_start();
   load_twiddles<N>(s_tw, tw);
+  wait_for_previous_kernel();
   const TElem* __restrict__ trow = static_cast<const TElem*>(t_origin) + (long)row * p_w;
   float2* prow = psi_item + (long)row * N;
   const RowLayout<N> L;
@@ -162,7 +164,9 @@ __device__ __forceinline__ void col_tile(float2* __restrict__ psi_item, const Co
   constexpr int nblk = N / G;
   const int j = threadIdx.x / G, g = threadIdx.x - j * G;
   const int c = cb * G + g;
+  let_next_kernel_start();
   load_twiddles<N>(s_tw, tw);
+  wait_for_previous_kernel();
   float2* base = psi_item + c;
   float2 v[P];
 #pragma unroll
