@@ -204,7 +204,8 @@ TOTEM_API int totem_transmission_run(const TotemStemArgs *args, TotemStemOut *ou
  *                      x phases direct: O(atoms x width + pixels log pixels), relative error
  *                      ~1e-7; used where the axes are uniform and the grid has at most 4096
  *                      rows, otherwise DIRECT is used.
- * ``scratch_bytes`` bounds the gridding work memory taken during a build (0 = 1 GiB); the arrays of
+ * ``scratch_bytes`` bounds the gridding work memory taken during a build (0 = 1 GiB; a quarter of it
+ * for each request of a server); the arrays of
  * one species of one slice (at most 64 bytes per pixel of the grid, its height rounded up to an edge of the
  * fused transforms) are always taken. */
 #define TOTEM_TX_AUTO 0
@@ -243,7 +244,8 @@ TOTEM_API int totem_inject_failures(long long alloc_after, int prepare_every);
  * Process-wide; no counterpart in the reference, which sizes its batch from free memory
  * (cuda_source_lobato.cu:1250-1260). */
 TOTEM_API int totem_load_tuning(const char *path, int *entries);
-/* The launch shapes a fused run on ``device`` with an n x n window would use by default. */
+/* The launch shapes a fused run on ``device`` with an n x n window would use by default (batch_bytes
+ * bounds the waves of one launch). */
 TOTEM_API int totem_tuned_config(int device, int n, int *row_variant, int *col_variant, long long *batch_bytes);
 /* The gridding builder's batch plan, without a device (tests): jobs are numbered in slice order,
  * slice s owning jobs [job_beg[s], job_beg[s+1]); at most jobs_per_batch jobs run per batch.

@@ -508,9 +508,14 @@ Status totem_session::build_transmission(int path, int* launches) {
       // jobs per batch from the budget for their work memory, at least one; a device that has no
       // room for it takes the direct sums, unless gridding was asked for
       const totem::GridBytes need = totem::grid_bytes(p_h, p_w, grid_half, grid_kmax, grid_job_beg_h.back(), grid_atoms);
-      const size_t room = std::max(totem::tx_gridding_scratch(), need.tables + need.per_job) - need.tables;
-      const size_t jobs = std::max(grid_job_beg_h.back(), 1);
-      bytes = need.tables + need.per_job * std::min(room / need.per_job, jobs);
+      // A server's requests build side by side from one pool: each takes a quarter, but the whole where
+      // a slice needs it, so that a request is split as it is alone (and rounds the same)
+      const size_t whole = std::max(totem::tx_gridding_scratch(), need.tables + need.per_job) - need.tables;
+      size_t jobs = std::max(grid_job_beg_h.back(), 1), per_slice = 1;
+      for (int k = 0; k < slices; ++k)
+        per_slice = std::max<size_t>(per_slice, grid_job_beg_h[k + 1] - grid_job_beg_h[k]);
+      if (grid_scratch.pool) jobs = std::min(jobs, std::max(whole / 4 / need.per_job, per_slice));
+      bytes = need.tables + need.per_job * std::min(whole / need.per_job, jobs);
       const Status st = grid_scratch.ensure(bytes);
       if (!st.ok()) {
         if (mode == TOTEM_TX_GRIDDING || st.code != TOTEM_ERR_OOM) return st;
