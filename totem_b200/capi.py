@@ -211,12 +211,12 @@ def _split(z):
     pair = z.reshape(-1).view(np.float64).reshape(-1, 2)
     re_, im_ = np.empty(z.shape), np.empty(z.shape)
     n = len(pair)
-    step = max(_SPLIT_GRAIN, -(-n // 8))
+    step = -(-n // 8) if n >= 8 * _SPLIT_GRAIN else max(n, 1)
 
     def copy(lo):
         re_.reshape(-1)[lo:lo + step] = pair[lo:lo + step, 0]
         im_.reshape(-1)[lo:lo + step] = pair[lo:lo + step, 1]
-    if n <= step:
+    if n <= step:  # too small for threads to pay
         copy(0)
     else:
         with futures.ThreadPoolExecutor(8) as pool:
