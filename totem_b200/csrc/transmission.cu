@@ -702,6 +702,12 @@ Status launch_tx_gridding(const TxGrid& g, const SpeciesSet& sp, const GridPlanD
     finish = false;
     batches = grid_batches(job_beg, per_batch);
   }
+  // The inverse row transform runs with each batch; where a batch's rows are no whole row tiles (2048 rows
+  // of 160 columns in batches of 111 slices: tiles of 20 rows) once after the last, over the whole stack,
+  // whose rows are (tx_fft_shape_ok).
+  bool rows_by_batch = true;
+  for (const GridBatch& b : batches)
+    if (finish && (long)(b.s_hi - b.s_lo) * g.p_h % tx_tiles_of(g.p_w).x) rows_by_batch = false;
   if (jobs > 0) {
     const size_t smem = sizeof(int) * (2 * (size_t)gp.n + 1);
     TOTEM_TRY(ensure_smem((const void*)k_grid_sort, smem));
@@ -728,9 +734,12 @@ Status launch_tx_gridding(const TxGrid& g, const SpeciesSet& sp, const GridPlanD
       float2* first = out + (long)b.s_lo * plane;
       TOTEM_TRY(TOTEM_GRID_DISPATCH(g.p_h, grid_cols_inv, grid_cols_inv, g, sp, gp, w, b.s_lo, b.s_hi, b.j_lo, out,
                                     tw_h, st));
-      TOTEM_TRY(TOTEM_GRID_DISPATCH(g.p_w, rows_exp, tx_rows_exp, first, (long)(b.s_hi - b.s_lo) * g.p_h, tw_w, sig,
-                                    st));
-      *launches += 2;
+      ++*launches;
+      if (rows_by_batch) {
+        TOTEM_TRY(TOTEM_GRID_DISPATCH(g.p_w, rows_exp, tx_rows_exp, first, (long)(b.s_hi - b.s_lo) * g.p_h, tw_w, sig,
+                                      st));
+        ++*launches;
+      }
       continue;
     }
     const unsigned cx = (unsigned)std::min<long>((plane + 255) / 256, 2048);
@@ -740,6 +749,10 @@ Status launch_tx_gridding(const TxGrid& g, const SpeciesSet& sp, const GridPlanD
       TOTEM_TRY(cuda_status(cudaGetLastError(), "k_grid_combine"));
       ++*launches;
     }
+  }
+  if (finish && !rows_by_batch) {
+    TOTEM_TRY(TOTEM_GRID_DISPATCH(g.p_w, rows_exp, tx_rows_exp, out, (long)g.slices * g.p_h, tw_w, sig, st));
+    ++*launches;
   }
   *finished = finish;
   return Status::Ok();
