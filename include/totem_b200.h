@@ -203,7 +203,7 @@ TOTEM_API int totem_transmission_run(const TotemStemArgs *args, TotemStemOut *ou
  *   TOTEM_TX_GRIDDING  gridding along y onto a twice-finer axis and FFTs (a non-uniform FFT), the
  *                      x phases direct: O(atoms x width + pixels log pixels), relative error
  *                      ~1e-7; used where the axes are uniform and the grid has at most 4096
- *                      rows, otherwise DIRECT is used.
+ *                      rows and 2^30 points, otherwise DIRECT is used.
  * ``scratch_bytes`` bounds the gridding work memory taken during a build (0 = 1 GiB; a quarter of it
  * for each request of a server); the arrays of
  * one species of one slice (at most 64 bytes per pixel of the grid, its height rounded up to an edge of the

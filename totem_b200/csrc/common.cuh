@@ -138,6 +138,12 @@ struct GridPlanDev {
   const int* job_beg = nullptr;    // [slices + 1] first job of every slice
   const int* atom_beg = nullptr;   // [jobs + 1] atoms of the jobs before
 };
+// Row pitch of the gridding builder's arrays: the columns formed (the half kx >= 0 and its last line, or
+// all p_w), rounded up to whole column tiles.
+inline long long grid_pitch(int p_w, int half) { return ((half ? p_w / 2 + 1LL : p_w) + 15) / 16 * 16; }
+// Whether the builder's kernels may take a grid of that width with transforms of n: they index a job's
+// 2 n fine rows (the largest of its arrays) by 32-bit integers.
+inline bool grid_indexes_fit(int n, int p_w, int half) { return 2LL * n * grid_pitch(p_w, half) <= 0x7fffffffLL; }
 // Work memory of the gridding builder (grid_work lays it out): tables of all jobs of the build, and
 // the large arrays of one batch of jobs.
 struct GridWork {

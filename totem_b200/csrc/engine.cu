@@ -576,8 +576,9 @@ Status totem_session::build_transmission(int path, int* launches) {
 
 // Uniform separable axes, kx(c) = kx0 + c dkx and ky(r) = ky0 + r dky (the reference's
 // meshgrid of (-P/2 : P/2-1) / (P dx), ToTEM_submit_v1.m:1534-1538), on a grid of up to 4096 rows
-// admit the gridding builder.  Its job table holds one job per species segment
-// of every slice (neutral, ionic, then the correction kinds), in slice order.
+// whose arrays the kernels can index (grid_indexes_fit) admit the gridding builder.  Its job table
+// holds one job per species segment of every slice (neutral, ionic, then the correction kinds), in
+// slice order.
 Status totem_session::plan_gridding(const TotemStemArgs* a, const totem::SpeciesHost* const (&kinds)[4]) {
   grid_ok = false;
   grid_job_beg_h.clear();
@@ -599,6 +600,7 @@ Status totem_session::plan_gridding(const TotemStemArgs* a, const totem::Species
   // S(-k) = conj S(k) column by column: kx antisymmetric about its middle column, ky centred
   grid_half = grid_sy == 0.0 && a->kx[p_w / 2] == 0.0;
   for (int c = 1; c < p_w / 2 && grid_half; ++c) grid_half = a->kx[p_w / 2 - c] == -a->kx[p_w / 2 + c];
+  if (!totem::grid_indexes_fit(grid_n, p_w, grid_half)) return Status::Ok();
   std::vector<int4> jobs;
   std::vector<int> atom_beg(1, 0);
   grid_job_beg_h.assign(slices + 1, 0);

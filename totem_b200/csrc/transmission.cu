@@ -517,7 +517,7 @@ size_t grid_work(int p_h, int p_w, int half, int kmax, int jobs, long long atoms
   w->kmax = kmax;
   w->half = half;
   w->cols = half ? p_w / 2 + 1 : p_w;
-  w->pitch = (w->cols + 15) / 16 * 16;
+  w->pitch = (int)grid_pitch(p_w, half);
   size_t off = 0;
   auto take = [&](size_t bytes) {
     char* p = base + off;
