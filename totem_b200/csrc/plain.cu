@@ -10,7 +10,8 @@
 //
 // The element-wise kernels are bound by memory: a grid row of blocks per item keeps the index
 // arithmetic to one 32-bit division (64-bit divisions per element made each of them two to three
-// times as long as its traffic takes).
+// times as long as its traffic takes).  The element index is unsigned: the step past the last element of
+// an item of nearly 2^31 is not negative.
 #include "common.cuh"
 
 namespace totem {
@@ -29,8 +30,8 @@ __global__ void __launch_bounds__(256) k_plain_gather_mul(float2* __restrict__ p
                        geo.begin_col + (pos % geo.width_red) * geo.step;
     float2* dst = psi + (long)item * vol;
     const float2* src = probe != nullptr ? probe + (long)(gi / geo.depth) * vol : dst;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < vol; e += gridDim.x * blockDim.x) {
-      const int r = e / w, c = e - r * w;
+    for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < (unsigned)vol; e += gridDim.x * blockDim.x) {
+      const unsigned r = e / (unsigned)w, c = e - r * w;
       const float2 t = tslice != nullptr ? __ldg(t0 + (long)r * geo.p_width + c) : make_float2(1.f, 0.f);
       const float2 u = src[e], v = make_float2(u.x * scale, u.y * scale);
       dst[e] = make_float2(v.x * t.x - v.y * t.y, v.x * t.y + v.y * t.x);
@@ -42,7 +43,7 @@ __global__ void __launch_bounds__(256) k_plain_mul(float2* __restrict__ psi, con
                                                    int items) {
   for (int item = blockIdx.y; item < items; item += gridDim.y) {
     float2* p = psi + (long)item * vol;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < vol; e += gridDim.x * blockDim.x) {
+    for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < (unsigned)vol; e += gridDim.x * blockDim.x) {
       const float2 t = __ldg(m + e), v = p[e];
       p[e] = make_float2(v.x * t.x - v.y * t.y, v.x * t.y + v.y * t.x);
     }
@@ -132,7 +133,7 @@ inline int grid_for(long total) { return (int)std::min<long>((total + 255) / 256
 
 // blocks of 256 threads along an item of vol elements (four elements each), items along y
 inline dim3 item_grid(int vol, int items) {
-  return dim3((unsigned)std::max(1, (vol + 1023) / 1024), (unsigned)std::min(items, 65535));
+  return dim3(std::max(1u, ((unsigned)vol + 1023) / 1024), (unsigned)std::min(items, 65535));
 }
 
 Status launch_plain_gather_mul(float2* psi, const float2* probe, const float2* tslice, int h, int w, int items,
