@@ -7,30 +7,30 @@
 #include <algorithm>
 #include <cstddef>
 #include <cstdlib>
+#include <exception>
 #include <memory>
 #include <new>
-#include <system_error>
 #include <thread>
-#include <vector>
 
 namespace totem {
 
 // f(lo, hi) over [0, n) in up to eight pieces of at least ``grain`` elements; f must not throw.
 template <class F>
 void host_parallel(size_t n, size_t grain, F&& f) {
+  constexpr size_t kMost = 8;
   const size_t hw = std::max(1u, std::thread::hardware_concurrency());
-  const size_t parts = std::max<size_t>(1, std::min<size_t>({8, hw, n / std::max<size_t>(1, grain)}));
+  const size_t parts = std::max<size_t>(1, std::min<size_t>({kMost, hw, n / std::max<size_t>(1, grain)}));
   const size_t step = (n + parts - 1) / parts;
-  std::vector<std::thread> threads;
-  threads.reserve(parts);
-  size_t lo = step;  // the caller takes the first piece
+  std::thread threads[kMost];  // (no container: nothing below may throw while one is running)
+  size_t lo = step;            // the caller takes the first piece
   try {
-    for (; lo < n; lo += step) threads.emplace_back([&f, lo, hi = std::min(n, lo + step)] { f(lo, hi); });
-  } catch (const std::system_error&) {
-    f(lo, n);  // no more threads to be had: the rest here
+    for (size_t i = 0; lo < n; lo += step, ++i) threads[i] = std::thread([&f, lo, hi = std::min(n, lo + step)] { f(lo, hi); });
+  } catch (const std::exception&) {  // no more threads, or no memory for one: the rest here
+    f(lo, n);
   }
   if (n > 0) f(0, std::min(n, step));
-  for (std::thread& t : threads) t.join();
+  for (std::thread& t : threads)
+    if (t.joinable()) t.join();
 }
 
 // An uninitialised host array (std::vector would write it twice).
