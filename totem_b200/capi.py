@@ -216,11 +216,16 @@ def _split(z):
     def copy(lo):
         re_.reshape(-1)[lo:lo + step] = pair[lo:lo + step, 0]
         im_.reshape(-1)[lo:lo + step] = pair[lo:lo + step, 1]
-    if n <= step:  # too small for threads to pay
-        copy(0)
-    else:
-        with futures.ThreadPoolExecutor(8) as pool:
-            list(pool.map(copy, range(0, n, step)))
+    blocks = range(0, n, step)
+    if len(blocks) > 1:  # fewer are too small for threads to pay
+        try:
+            with futures.ThreadPoolExecutor(8) as pool:
+                list(pool.map(copy, blocks))
+            return re_, im_
+        except RuntimeError:  # no thread to be had (a limit, or an interpreter that is shutting down)
+            pass
+    for lo in blocks:
+        copy(lo)
     return re_, im_
 
 
