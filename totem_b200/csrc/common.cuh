@@ -46,7 +46,9 @@ cudaError_t launch_kernel(void (*kernel)(Params...), unsigned grid, unsigned blo
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = overlap ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();  // returned here: not left for the next launch's check to find
+  return e;
 }
 
 #define TOTEM_CUDA(call)                                              \
