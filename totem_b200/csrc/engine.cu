@@ -902,7 +902,7 @@ Status totem_session::slice_loop(int path, int batch, bool batch_fixed, int col_
       key.push_back((long long)(uintptr_t)q);
     key.insert(key.end(), event_of_slice.begin(), event_of_slice.end());
     key.insert(key.end(), de.layer_event.begin(), de.layer_event.end());
-    TOTEM_TRY(run_graphed(key, enqueue, launches));
+    TOTEM_TRY(run_graphed(stem_graph, key, enqueue, launches));
   }
   has_result = true;
   return Status::Ok();
@@ -914,20 +914,20 @@ Status totem_session::slice_loop(int path, int batch, bool batch_fixed, int col_
 // with a new key executes directly (it also sets every kernel's shared-memory limit, which is
 // not done during capture).  Streams that cannot be captured (the legacy default stream, or one
 // the caller is capturing already) run directly.
-Status totem_session::run_graphed(const std::vector<long long>& key, const std::function<Status()>& enqueue,
-                                  int* launches) {
+Status totem_session::run_graphed(LoopGraph& graph, const std::vector<long long>& key,
+                                  const std::function<Status()>& enqueue, int* launches) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   const bool capturable = stream != nullptr && stream != cudaStreamLegacy && stream != cudaStreamPerThread &&
                           cudaStreamIsCapturing(stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
   if (!capturable) return enqueue();
-  if (graph_exec != nullptr && key == graph_key) {
-    TOTEM_CUDA(cudaGraphLaunch(graph_exec, stream));
-    *launches += graph_launches;
+  if (graph.exec != nullptr && key == graph.key) {
+    TOTEM_CUDA(cudaGraphLaunch(graph.exec, stream));
+    *launches += graph.launches;
     return Status::Ok();
   }
-  if (key != graph_key) {  // first run of this shape
-    drop_graph();
-    graph_key = key;
+  if (key != graph.key) {  // first run of this shape
+    graph.drop();
+    graph.key = key;
     return enqueue();
   }
   const int before = *launches;
@@ -937,26 +937,20 @@ Status totem_session::run_graphed(const std::vector<long long>& key, const std::
   const cudaError_t e = cudaStreamEndCapture(stream, &g);
   if (!st.ok() || e != cudaSuccess) {
     if (g) cudaGraphDestroy(g);
-    graph_key.clear();
+    graph.key.clear();
     return st.ok() ? totem::cuda_status(e, "cudaStreamEndCapture") : st;
   }
   cudaGraphExec_t x = nullptr;
   const cudaError_t ei = cudaGraphInstantiate(&x, g, 0);
   cudaGraphDestroy(g);
   if (ei != cudaSuccess) {
-    graph_key.clear();
+    graph.key.clear();
     return totem::cuda_status(ei, "cudaGraphInstantiate");
   }
-  graph_exec = x;
-  graph_launches = *launches - before;
-  TOTEM_CUDA(cudaGraphLaunch(graph_exec, stream));
+  graph.exec = x;
+  graph.launches = *launches - before;
+  TOTEM_CUDA(cudaGraphLaunch(graph.exec, stream));
   return Status::Ok();
-}
-
-void totem_session::drop_graph() {
-  if (graph_exec) cudaGraphExecDestroy(graph_exec);
-  graph_exec = nullptr;
-  graph_launches = 0;
 }
 
 totem::DetectionEvents totem_session::detection_events() const {
@@ -994,7 +988,8 @@ Status totem_session::combine_results(const totem::DetectionEvents& de, int* lau
 
 // The slice loop of HRTEM and CBED: every pass on ``s`` from its probe, the last slice's spectrum kept
 // in psi.  Few waves and many short launches: a repeated call replays them as one graph.
-Status totem_session::spectrum_loop(totem::SliceLoopArgs s, const char* t, size_t tslice_bytes, int* launches) {
+Status totem_session::spectrum_loop(LoopGraph& graph, totem::SliceLoopArgs s, const char* t, size_t tslice_bytes,
+                                    int* launches) {
   s.overlap = overlap_pays(s.n) ? 1 : 0;
   auto enqueue = [&]() -> Status {
     TOTEM_TRY(totem::launch_row_pass(s, t, true, stream));
@@ -1006,13 +1001,13 @@ Status totem_session::spectrum_loop(totem::SliceLoopArgs s, const char* t, size_
     return Status::Ok();
   };
   if (!totem::slice_graphs_enabled()) return enqueue();
-  // what the launches embed (the first entry tells them from the detectors' loop)
-  std::vector<long long> key = {-1, s.n, s.items, slices, (long long)tslice_bytes, s.p_h, s.t_bf16, s.skip_band,
+  // what the launches embed
+  std::vector<long long> key = {s.n, s.items, slices, (long long)tslice_bytes, s.p_h, s.t_bf16, s.skip_band,
                                 s.skip_rows, s.geo.begin_row, s.geo.begin_col, s.geo.step, s.geo.width_red, s.geo.depth,
                                 s.geo.p_width};
   for (const void* q : {(const void*)s.psi, (const void*)s.probe, (const void*)s.prop, (const void*)s.tw, (const void*)t})
     key.push_back((long long)(uintptr_t)q);
-  return run_graphed(key, enqueue, launches);
+  return run_graphed(graph, key, enqueue, launches);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1075,7 +1070,7 @@ Status totem_session::hrtem(const TotemHrtemArgs* hr, TotemHrtemOut* out) {
   }
   // psi = wave .* T_0, then per slice FFT2 .* psf_fft IFFT2 .* T_{k+1}; the last column pass keeps
   // the spectrum FFT2(psi_{S-1} .* T) .* psf_fft, whose IFFT2 is the exit wave
-  TOTEM_TRY(spectrum_loop(s, static_cast<const char*>(Tslices), tslice_bytes, &launches));
+  TOTEM_TRY(spectrum_loop(hrtem_graph, s, static_cast<const char*>(Tslices), tslice_bytes, &launches));
   const float2* spec = psi.as<float2>();
   const bool want_exit = out && (out->exit_re || out->exit_im);
   const bool want_img = out && out->image && hr->defoci > 0;
@@ -1192,7 +1187,7 @@ Status totem_session::cbed(double* pattern) {
     s.tw = tw_n.as<float2>(); s.aper_num = 0;
     s.skip_band = (totem::band_skip_enabled() && totem::band_skip_ok(h, band, 0)) ? 1 : 0;
     s.skip_rows = (totem::band_skip_enabled() && totem::band_rows_ok(h, row_band)) ? 1 : 0;
-    TOTEM_TRY(spectrum_loop(s, reinterpret_cast<const char*>(Tp), plane * sizeof(float2), &launches));
+    TOTEM_TRY(spectrum_loop(cbed_graph, s, reinterpret_cast<const char*>(Tp), plane * sizeof(float2), &launches));
   } else {
     cufftHandle p;
     TOTEM_TRY(plan(h, w, w_num, &p));

@@ -232,10 +232,19 @@ struct totem_session {
   bool has_result = false;
   int last_what = 0;
   std::map<totem::PlanKey, cufftHandle> plans;
-  // the fused slice loop of the last run, as a CUDA graph (run_graphed)
-  std::vector<long long> graph_key;
-  cudaGraphExec_t graph_exec = nullptr;
-  int graph_launches = 0;
+  // the last fused slice loop of each kind, as a CUDA graph (run_graphed); one per kind, so that calls of
+  // one leave those of another in place
+  struct LoopGraph {
+    std::vector<long long> key;
+    cudaGraphExec_t exec = nullptr;
+    int launches = 0;
+    void drop() {
+      if (exec) cudaGraphExecDestroy(exec);
+      exec = nullptr;
+      launches = 0;
+    }
+  };
+  LoopGraph stem_graph, cbed_graph, hrtem_graph;
 
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
   TotemTiming timing{};
@@ -255,7 +264,7 @@ struct totem_session {
     // buffers first: pool-backed ones are freed in order on ``stream``, which must still exist
     for_each_buf([](totem::DevBuf& b) { b.release(); });
     for (auto& kv : plans) cufftDestroy(kv.second);
-    drop_graph();
+    for (LoopGraph* g : {&stem_graph, &cbed_graph, &hrtem_graph}) g->drop();
     for (auto& e : ev)
       if (e) cudaEventDestroy(e);
     for (auto& e : pev) cudaEventDestroy(e);
@@ -336,9 +345,9 @@ struct totem_session {
   Status second_stream();
   // The transmission slices as the slice loop reads them (complex64, or bfloat16 pairs).
   Status transmission_for(int t_storage, const void** t, size_t* slice_bytes, int* launches);
-  Status run_graphed(const std::vector<long long>& key, const std::function<Status()>& enqueue, int* launches);
-  void drop_graph();
-  Status spectrum_loop(totem::SliceLoopArgs s, const char* t, size_t tslice_bytes, int* launches);
+  Status run_graphed(LoopGraph& graph, const std::vector<long long>& key, const std::function<Status()>& enqueue,
+                     int* launches);
+  Status spectrum_loop(LoopGraph& graph, totem::SliceLoopArgs s, const char* t, size_t tslice_bytes, int* launches);
   Status hrtem(const TotemHrtemArgs* h, TotemHrtemOut* out);
   Status hrtem_plain(const TotemHrtemArgs* hr, TotemHrtemOut* out, const float2* Tp);
   Status cbed(double* pattern);
