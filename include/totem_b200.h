@@ -205,9 +205,10 @@ TOTEM_API int totem_transmission_run(const TotemStemArgs *args, TotemStemOut *ou
  *                      ~1e-7; used where the axes are uniform and the grid has at most 4096
  *                      rows and 2^30 points, otherwise DIRECT is used.
  * ``scratch_bytes`` bounds the gridding work memory taken during a build (0 = 1 GiB; a quarter of it
- * for each request of a server); the arrays of
- * one species of one slice (at most 64 bytes per pixel of the grid, its height rounded up to an edge of the
- * fused transforms) are always taken. */
+ * for each request of a server).  Beyond the bound if need be, a build always takes 48 bytes per atom
+ * and 9 n bytes per species of a slice, and the arrays of one species of one slice: at most 64 bytes
+ * per pixel of an n x m grid (half of that where both axes are centred on zero), where n is its height
+ * rounded up to an edge of the fused transforms and m its width rounded up to 16. */
 #define TOTEM_TX_AUTO 0
 #define TOTEM_TX_DIRECT 1
 #define TOTEM_TX_GRIDDING 2

@@ -1,0 +1,56 @@
+"""Work memory of the gridding transmission builder for slices of many atoms: bounded by the grid and a few
+tables per atom, the phases held in pieces of columns and of atoms, with the same numbers bit by bit."""
+from dataclasses import replace
+
+import numpy as np
+import pytest
+
+from tests.conftest import rel_l2
+from tests.test_gpu_gridding_edges import _both, _request
+from totem_b200 import capi
+
+pytestmark = pytest.mark.gpu
+TOL = 5e-6  # the gridding edge tests' bound against the direct sums: the FP32 rounding both share
+
+
+def _sparse(req, occupancy):
+    """The same rows at a small occupancy, so that many atoms make no more potential than a few."""
+    rows = req.ele_n.copy()
+    rows[:, 2] *= occupancy
+    return replace(req, ele_n=rows)
+
+
+@pytest.mark.parametrize("p_h,p_w,atoms,kw", [
+    (64, 64, 1500, {}),                                      # six pieces of 256 groups
+    (64, 30, 700, {"centred": False}),                       # a pitch below 128 columns
+    (64, 512, 3000, {}),                                     # three pieces of columns by six of groups
+    (96, 96, 5000, {"equal_y": True, "flag": "l"}),          # groups of eight atoms
+    (62, 200, 2000, {"centred": False}),
+])
+def test_phases_in_pieces_change_no_bit(engine_lib, p_h, p_w, atoms, kw):
+    req = _sparse(_request(p_h, p_w, atoms, **kw), 50.0 / atoms)
+    direct, whole = _both(req, 0)
+    _, pieces = _both(req, 1)
+    assert rel_l2(whole, direct) < TOL and rel_l2(whole - 1.0, direct - 1.0) < 20 * TOL
+    assert rel_l2(pieces, whole) < 1e-6  # a slice's two species through memory
+    one = replace(req, ele_n=np.concatenate([req.ele_n[2 * atoms * k:][:atoms] for k in range(req.slices)]),
+                  series_n=np.full(req.slices, float(atoms)))
+    assert np.array_equal(_both(one, 1)[1], _both(one, 0)[1])
+
+
+def test_memory_does_not_grow_with_a_kilobyte_per_atom(engine_lib):
+    import torch
+    atoms = 200_000
+    req = _sparse(_request(64, 64, atoms, slices=1), 1e-4)
+    torch.cuda.synchronize()
+    with capi.tx_builder(capi.TX_GRIDDING, 1 << 20):
+        s = capi.Session(device=0)
+        s.upload(req, stem=False)
+        free = torch.cuda.mem_get_info()[0]
+        s.run(what=1)
+        s.download()
+        taken = free - torch.cuda.mem_get_info()[0]
+        s.close()
+    # 48 bytes an atom of the two species, 64 a pixel and the transmission itself; 64 MB for what the
+    # driver keeps (a kilobyte an atom were 205 MB)
+    assert taken < 2 * atoms * 48 + 64 * 64 * 72 + (64 << 20), taken

@@ -162,7 +162,8 @@ struct GridWork {
   unsigned char* used = nullptr;   // [jobs][2 n / 16]: a group spreads into this block of fine rows
   // one batch
   int ex_cols = 0;                 // columns of E held at a time (a multiple of 128, or pitch)
-  float2* ex = nullptr;            // [jobs][kmax][ex_cols]
+  int ex_rows = 0;                 // groups of E held at a time (kmax, or fewer)
+  float2* ex = nullptr;            // [jobs][ex_rows][ex_cols]
   float2* fine = nullptr;          // [jobs][2 n][pitch]
   float2* s = nullptr;             // [jobs][p_h + 1][pitch]
 };
@@ -170,17 +171,21 @@ struct GridBatch {
   int s_lo, s_hi, j_lo, j_hi;
 };
 std::vector<GridBatch> grid_batches(const std::vector<int>& job_beg, int jobs_per_batch);
-// Work memory: bytes of the tables of all jobs, and of one job's large arrays in a batch.
+// Work memory: bytes of the tables of all jobs, and of one job's large arrays in a batch, which hold the
+// phases of ``ex_rows`` of its at most kmax atoms at a time.
 struct GridBytes {
   size_t tables, per_job;
 };
-GridBytes grid_bytes(int p_h, int p_w, int half, int kmax, int jobs, long long atoms);
+GridBytes grid_bytes(int p_h, int p_w, int half, int kmax, int ex_rows, int jobs, long long atoms);
+// ex_rows for which a job's large arrays take ``job_bytes``; not below what makes the phases as large as
+// 4 p_h rows, and not above kmax.
+int grid_piece_rows(int p_h, int p_w, int half, int kmax, size_t job_bytes);
 // Overwrites out like launch_tx_species; ``scratch`` holds the tables and at least one job's arrays.
 // With ``finish`` (the transmission's fused FFT takes the grid and nothing is to be added to V) out
 // receives T = exp(i sig V) of every slice and *finished is set, unless a slice has more jobs than a
 // batch holds.
 Status launch_tx_gridding(const TxGrid& g, const SpeciesSet& sp, const GridPlanDev& gp,
-                          const std::vector<int>& job_beg, int kmax, long long atoms, const float2* tw_w,
+                          const std::vector<int>& job_beg, int kmax, int ex_rows, long long atoms, const float2* tw_w,
                           const float2* tw_h, void* scratch, size_t scratch_bytes, bool finish, float sig, float2* out,
                           cudaStream_t st, int* launches, bool* finished);
 // The smallest edge of the fused transforms that is at least p_h; 0 if there is none.

@@ -504,16 +504,25 @@ Status totem_session::build_transmission(int path, int* launches) {
     const int mode = totem::tx_builder_mode();
     bool gridding = grid_ok && (mode == TOTEM_TX_GRIDDING || (mode == TOTEM_TX_AUTO && gridding_cheaper()));
     size_t bytes = 0;
+    int ex_rows = grid_kmax;
     if (gridding) {
       // jobs per batch from the budget for their work memory, at least one; a device that has no
       // room for it takes the direct sums, unless gridding was asked for
-      const totem::GridBytes need = totem::grid_bytes(p_h, p_w, grid_half, grid_kmax, grid_job_beg_h.back(), grid_atoms);
-      // A server's requests build side by side from one pool: each takes a quarter, but the whole where
-      // a slice needs it, so that a request is split as it is alone (and rounds the same)
-      const size_t whole = std::max(totem::tx_gridding_scratch(), need.tables + need.per_job) - need.tables;
-      size_t jobs = std::max(grid_job_beg_h.back(), 1), per_slice = 1;
+      const int all = grid_job_beg_h.back();
+      size_t jobs = std::max(all, 1), per_slice = 1;
       for (int k = 0; k < slices; ++k)
         per_slice = std::max<size_t>(per_slice, grid_job_beg_h[k + 1] - grid_job_beg_h[k]);
+      // the phases of a species' atoms in pieces where a slice's arrays would not keep to the budget
+      const size_t limit = totem::tx_gridding_scratch();
+      totem::GridBytes need = totem::grid_bytes(p_h, p_w, grid_half, grid_kmax, ex_rows, all, grid_atoms);
+      if (need.tables + need.per_job * per_slice > limit) {
+        ex_rows = totem::grid_piece_rows(p_h, p_w, grid_half, grid_kmax,
+                                         limit > need.tables ? (limit - need.tables) / per_slice : 0);
+        need = totem::grid_bytes(p_h, p_w, grid_half, grid_kmax, ex_rows, all, grid_atoms);
+      }
+      // A server's requests build side by side from one pool: each takes a quarter, but the whole where
+      // a slice needs it, so that a request is split as it is alone (and rounds the same)
+      const size_t whole = std::max(limit, need.tables + need.per_job) - need.tables;
       if (grid_scratch.pool) jobs = std::min(jobs, std::max(whole / 4 / need.per_job, per_slice));
       bytes = need.tables + need.per_job * std::min(whole / need.per_job, jobs);
       const Status st = grid_scratch.ensure(bytes);
@@ -531,7 +540,7 @@ Status totem_session::build_transmission(int path, int* launches) {
       gp.atom_beg = grid_atom_beg.as<int>();
       ran_tx_builder = TOTEM_TX_GRIDDING;
       const bool finish = path != TOTEM_PATH_PLAIN && fft_fused && (corr_by_species || !(vcn.beg || vci.beg));
-      TOTEM_TRY(totem::launch_tx_gridding(g, set, gp, grid_job_beg_h, grid_kmax, grid_atoms, tw_pw.as<float2>(),
+      TOTEM_TRY(totem::launch_tx_gridding(g, set, gp, grid_job_beg_h, grid_kmax, ex_rows, grid_atoms, tw_pw.as<float2>(),
                                           tw_ph.as<float2>(), grid_scratch.p, bytes, finish, sig, T.as<float2>(),
                                           stream, launches, &finished));
       // work memory of the build only: returned at once to a server's pool (stream-ordered and

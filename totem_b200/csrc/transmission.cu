@@ -387,24 +387,25 @@ __global__ void __launch_bounds__(GR_T) k_grid_sort(GridPlanDev gp, SpeciesSet s
 }
 
 // E[group][column]: the direct x phases, summed over the group's atoms, and the groups' spreading
-// weights.  A CTA takes 128 columns of every gridDim.y-th chunk of 16 groups of one job.
+// weights, for the groups [g0, g0 + ex_rows).  A CTA takes 128 columns of every gridDim.y-th chunk of 16
+// groups of one job.
 __global__ void __launch_bounds__(128) k_grid_phases(GridPlanDev gp, SpeciesSet spset, TxGrid g, int job0,
-                                                     int col0, GridWork w) {
+                                                     int col0, int g0, GridWork w) {
   const int h = col0 + blockIdx.x * 128 + threadIdx.x, job = job0 + blockIdx.z;
   const int4 jb = gp.jobs[job];
   const double* pos = spset.k[jb.x & 3].pos + 2L * jb.z;
   const int* order = w.order + gp.atom_beg[job];
   const int* first = w.first + gp.atom_beg[job] + job;
   float* wgt = reinterpret_cast<float*>(w.wgt + 2L * gp.atom_beg[job]);
-  float2* ex = w.ex + (long)blockIdx.z * w.kmax * w.ex_cols + (h - col0);
-  const int groups = w.groups[job];
+  float2* ex = w.ex + (long)blockIdx.z * w.ex_rows * w.ex_cols + (h - col0);
+  const int groups = min(w.groups[job], g0 + w.ex_rows);
   // half: column h holds kx = h dkx, the last of them +p_w / 2 (the grid's own -p_w / 2 is its
   // conjugate); columns beyond ``cols`` pad the pitch
   const double kx = h >= w.cols ? 0.0
                     : !w.half   ? g.kx_axis[h]
                     : 2 * h < g.p_w ? g.kx_axis[g.p_w / 2 + h]
                                     : -g.kx_axis[0];
-  for (int q0 = blockIdx.y * 16; q0 < groups; q0 += gridDim.y * 16) {
+  for (int q0 = g0 + blockIdx.y * 16; q0 < groups; q0 += gridDim.y * 16) {
     if (h < 128) {  // thread (q, k): weight k of group q
       const int q = q0 + threadIdx.x / GR_W, k = threadIdx.x % GR_W;
       if (q < groups) {
@@ -420,7 +421,7 @@ __global__ void __launch_bounds__(128) k_grid_phases(GridPlanDev gp, SpeciesSet 
         const double* p = pos + 2L * order[i];
         s = cadd(s, phase_of(kx * p[0] + (w.half ? 0.0 : gp.sy * p[1])));
       }
-      ex[(long)q * w.ex_cols] = s;
+      ex[(long)(q - g0) * w.ex_cols] = s;
     }
   }
 }
@@ -436,8 +437,11 @@ __device__ __forceinline__ void spread_at(float2 (&acc)[GR_ROWS], const float* w
 // One block of GR_ROWS fine rows of one job and 128 columns, a column per thread: the groups that
 // reach the block in sorted order.  All lanes take the same group, so its offset picks one of the 23
 // unrolled bodies without divergence and the weights are uniform loads; E is loaded four groups
-// ahead of its use.
-__global__ void __launch_bounds__(128) k_grid_spread(GridPlanDev gp, int job0, int col0, GridWork w) {
+// ahead of its use.  PIECES: of the groups only [g0, g0 + ex_rows) are held: from the second such piece on the
+// sums continue from the rows in memory, in the same order (the groups that wrap around sort last), so
+// the pieces change no bit.
+template <bool PIECES>
+__global__ void __launch_bounds__(128) k_grid_spread(GridPlanDev gp, int job0, int col0, int g0, GridWork w) {
   const int nf = 2 * gp.n, f0 = blockIdx.y * GR_ROWS, job = job0 + blockIdx.z;
   const int h = col0 + blockIdx.x * 128 + threadIdx.x;
   if (!w.used[(long)job * (nf / GR_ROWS) + blockIdx.y]) return;
@@ -445,12 +449,17 @@ __global__ void __launch_bounds__(128) k_grid_spread(GridPlanDev gp, int job0, i
   const int* __restrict__ ptr = w.ptr + (long)job * (nf + 1);
   const int* __restrict__ base = w.base + gp.atom_beg[job];
   const float4* __restrict__ wgt = w.wgt + 2L * gp.atom_beg[job];
-  const float2* __restrict__ ex = w.ex + (long)blockIdx.z * w.kmax * w.ex_cols + (hc - col0);
+  const float2* __restrict__ ex = w.ex + ((long)blockIdx.z * w.ex_rows - (PIECES ? g0 : 0)) * w.ex_cols + (hc - col0);
+  float2* dst = w.fine + ((long)blockIdx.z * nf + f0) * w.pitch + hc;
   float2 acc[GR_ROWS];
 #pragma unroll
-  for (int t = 0; t < GR_ROWS; ++t) acc[t] = make_float2(0.f, 0.f);
-  for (int wrap = f0 == 0 ? 1 : 0; wrap >= 0; --wrap) {
-    const int lo = ptr[wrap ? nf - GR_W + 1 : max(f0 - GR_W + 1, 0)], hi = ptr[wrap ? nf : f0 + GR_ROWS];
+  for (int t = 0; t < GR_ROWS; ++t) acc[t] = PIECES && g0 > 0 ? dst[(long)t * w.pitch] : make_float2(0.f, 0.f);
+  for (int wrap = 0; wrap <= (f0 == 0 ? 1 : 0); ++wrap) {
+    int lo = ptr[wrap ? nf - GR_W + 1 : max(f0 - GR_W + 1, 0)], hi = ptr[wrap ? nf : f0 + GR_ROWS];
+    if (PIECES) {
+      lo = max(lo, g0);
+      hi = min(hi, g0 + w.ex_rows);
+    }
     const int shift = (wrap ? nf : 0) + f0;
     for (int q0 = lo; q0 < hi; q0 += 4) {
       float2 x[4];
@@ -474,7 +483,6 @@ __global__ void __launch_bounds__(128) k_grid_spread(GridPlanDev gp, int job0, i
     }
   }
   if (h >= w.pitch) return;
-  float2* dst = w.fine + ((long)blockIdx.z * nf + f0) * w.pitch + h;
 #pragma unroll
   for (int t = 0; t < GR_ROWS; ++t) dst[(long)t * w.pitch] = acc[t];
 }
@@ -510,9 +518,17 @@ __global__ void __launch_bounds__(256) k_grid_combine(TxGrid g, SpeciesSet spset
   }
 }
 
+// Columns of E held at a time: all, or as many whole 128s as keep a row for each of kmax atoms within 4 p_h
+// rows (at least 128).
+int grid_ex_cols(int p_h, int pitch, int kmax) {
+  const long long cols = 4LL * p_h * pitch / kmax / 128 * 128;
+  return (int)std::min<long long>(pitch, std::max(cols, 128LL));
+}
+
 // Where the parts of the work memory lie (base may be null: sizes only); returns its bytes.
 // ``batch`` jobs in a batch.
-size_t grid_work(int p_h, int p_w, int half, int kmax, int jobs, long long atoms, int batch, char* base, GridWork* w) {
+size_t grid_work(int p_h, int p_w, int half, int kmax, int ex_rows, int jobs, long long atoms, int batch, char* base,
+                 GridWork* w) {
   const size_t n = grid_transform(p_h);
   w->kmax = kmax;
   w->half = half;
@@ -533,10 +549,10 @@ size_t grid_work(int p_h, int p_w, int half, int kmax, int jobs, long long atoms
   w->ptr = reinterpret_cast<int*>(take(nj * (2 * n + 1) * sizeof(int)));
   w->groups = reinterpret_cast<int*>(take(nj * sizeof(int)));
   w->used = reinterpret_cast<unsigned char*>(take(nj * (2 * n / GR_ROWS)));
-  // E is at most as large as two fine columns' worth of rows; jobs of more atoms take it in pieces
-  const long room = 4L * p_h * w->pitch / kmax / 128 * 128;
-  w->ex_cols = room >= w->pitch ? w->pitch : (int)std::max(room, 128L);
-  w->ex = reinterpret_cast<float2*>(take(nb * kmax * w->ex_cols * sizeof(float2)));
+  // E: ``ex_rows`` groups, in pieces of columns where the largest job's atoms would be more than 4 p_h rows
+  w->ex_cols = grid_ex_cols(p_h, w->pitch, kmax);
+  w->ex_rows = ex_rows;
+  w->ex = reinterpret_cast<float2*>(take(nb * w->ex_rows * w->ex_cols * sizeof(float2)));
   w->fine = reinterpret_cast<float2*>(take(nb * 2 * n * row));
   w->s = reinterpret_cast<float2*>(take(nb * (p_h + 1) * row));
   return off;
@@ -636,11 +652,19 @@ std::vector<float2> grid_deconvolution(int p_h, int n) {
   return t;
 }
 
-GridBytes grid_bytes(int p_h, int p_w, int half, int kmax, int jobs, long long atoms) {
+GridBytes grid_bytes(int p_h, int p_w, int half, int kmax, int ex_rows, int jobs, long long atoms) {
   GridWork w;
-  const size_t tables = grid_work(p_h, p_w, half, kmax, jobs, atoms, 0, nullptr, &w);
+  const size_t tables = grid_work(p_h, p_w, half, kmax, ex_rows, jobs, atoms, 0, nullptr, &w);
   // (each part of a batch is rounded up to 256 bytes as a whole, so the batch never needs more)
-  return GridBytes{tables, grid_work(p_h, p_w, half, kmax, jobs, atoms, 1, nullptr, &w) - tables};
+  return GridBytes{tables, grid_work(p_h, p_w, half, kmax, ex_rows, jobs, atoms, 1, nullptr, &w) - tables};
+}
+
+int grid_piece_rows(int p_h, int p_w, int half, int kmax, size_t job_bytes) {
+  const size_t rest = grid_bytes(p_h, p_w, half, kmax, 0, 1, 0).per_job;
+  const int pitch = (int)grid_pitch(p_w, half), cols = grid_ex_cols(p_h, pitch, kmax);
+  const long long least = std::max(64LL, 4LL * p_h * pitch / cols);
+  const long long room = job_bytes > rest ? (long long)((job_bytes - rest) / (cols * sizeof(float2))) : 0;
+  return (int)std::min<long long>(kmax, std::max(least, room));
 }
 
 std::vector<GridBatch> grid_batches(const std::vector<int>& job_beg, int jobs_per_batch) {
@@ -682,7 +706,7 @@ namespace {
 }  // namespace
 
 Status launch_tx_gridding(const TxGrid& g, const SpeciesSet& sp, const GridPlanDev& gp,
-                          const std::vector<int>& job_beg, int kmax, long long atoms, const float2* tw_w,
+                          const std::vector<int>& job_beg, int kmax, int ex_rows, long long atoms, const float2* tw_w,
                           const float2* tw_h, void* scratch, size_t scratch_bytes, bool finish, float sig, float2* out,
                           cudaStream_t st, int* launches, bool* finished) {
   *finished = false;
@@ -690,12 +714,12 @@ Status launch_tx_gridding(const TxGrid& g, const SpeciesSet& sp, const GridPlanD
   if ((int)job_beg.size() != g.slices + 1) return Status::Err(TOTEM_ERR_STATE, "gridding job table size");
   const long plane = (long)g.p_h * g.p_w;
   const int jobs = job_beg.back();
-  const GridBytes need = grid_bytes(g.p_h, g.p_w, gp.half, kmax, jobs, atoms);
+  const GridBytes need = grid_bytes(g.p_h, g.p_w, gp.half, kmax, ex_rows, jobs, atoms);
   if (scratch_bytes < need.tables + need.per_job) return Status::Err(TOTEM_ERR_STATE, "gridding scratch below one job");
   // at most 65535: the job is a grid dimension
   const int per_batch = (int)std::min<size_t>((scratch_bytes - need.tables) / need.per_job, 65535);
   GridWork w;
-  grid_work(g.p_h, g.p_w, gp.half, kmax, jobs, atoms, per_batch, static_cast<char*>(scratch), &w);
+  grid_work(g.p_h, g.p_w, gp.half, kmax, ex_rows, jobs, atoms, per_batch, static_cast<char*>(scratch), &w);
   std::vector<GridBatch> batches;
   if (finish) batches = whole_slice_batches(job_beg, per_batch);
   if (batches.empty()) {
@@ -720,12 +744,16 @@ Status launch_tx_gridding(const TxGrid& g, const SpeciesSet& sp, const GridPlanD
     if (nj > 0) {
       for (int col0 = 0; col0 < w.pitch; col0 += w.ex_cols) {
         const unsigned cx = (std::min(w.ex_cols, w.pitch - col0) + 127) / 128;
-        k_grid_phases<<<dim3(cx, (unsigned)std::min((kmax + 15) / 16, 1024), nj), 128, 0, st>>>(gp, sp, g, b.j_lo,
-                                                                                               col0, w);
-        TOTEM_TRY(cuda_status(cudaGetLastError(), "k_grid_phases"));
-        k_grid_spread<<<dim3(cx, 2 * gp.n / GR_ROWS, nj), 128, 0, st>>>(gp, b.j_lo, col0, w);
-        TOTEM_TRY(cuda_status(cudaGetLastError(), "k_grid_spread"));
-        *launches += 2;
+        for (int g0 = 0; g0 < kmax; g0 += w.ex_rows) {
+          const int ng = std::min(w.ex_rows, kmax - g0);
+          k_grid_phases<<<dim3(cx, (unsigned)std::min((ng + 15) / 16, 1024), nj), 128, 0, st>>>(gp, sp, g, b.j_lo, col0,
+                                                                                               g0, w);
+          TOTEM_TRY(cuda_status(cudaGetLastError(), "k_grid_phases"));
+          (w.ex_rows < kmax ? k_grid_spread<true> : k_grid_spread<false>)<<<dim3(cx, 2 * gp.n / GR_ROWS, nj), 128, 0, st>>>(
+              gp, b.j_lo, col0, g0, w);
+          TOTEM_TRY(cuda_status(cudaGetLastError(), "k_grid_spread"));
+          *launches += 2;
+        }
       }
       TOTEM_TRY(TOTEM_GRID_DISPATCH(gp.n, grid_cols, grid_cols, w, b.j_lo, nj, g.p_h, gp.ay, gp.tw, st));
       ++*launches;
