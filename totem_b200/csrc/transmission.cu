@@ -720,8 +720,9 @@ Status launch_tx_gridding(const TxGrid& g, const SpeciesSet& sp, const GridPlanD
   const int per_batch = (int)std::min<size_t>((scratch_bytes - need.tables) / need.per_job, 65535);
   GridWork w;
   grid_work(g.p_h, g.p_w, gp.half, kmax, ex_rows, jobs, atoms, per_batch, static_cast<char*>(scratch), &w);
-  std::vector<GridBatch> batches;
-  if (finish) batches = whole_slice_batches(job_beg, per_batch);
+  // whole slices in every batch: their sums do not depend on the batch size.  Where a batch does not hold
+  // a slice, its later jobs add to what the earlier ones wrote.
+  std::vector<GridBatch> batches = whole_slice_batches(job_beg, per_batch);
   if (batches.empty()) {
     finish = false;
     batches = grid_batches(job_beg, per_batch);
