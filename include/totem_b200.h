@@ -198,17 +198,19 @@ TOTEM_API int totem_transmission_run(const TotemStemArgs *args, TotemStemOut *ou
 /* How the neutral and ionic potential sums are formed on separable reciprocal grids (the
  * reference's meshgrid layout).  Process-wide; later transmission builds use it.  No
  * counterpart in the reference, whose cal_p sums every atom at every pixel.
- *   TOTEM_TX_AUTO      the cheaper of the two by a cost model (default)
+ *   TOTEM_TX_AUTO      the cheaper of the two by a cost model (default); DIRECT, slower and rounded
+ *                      otherwise, where the device has no room left even for the gridding of one slice
  *   TOTEM_TX_DIRECT    per-species sums over atoms at every pixel: O(atoms x pixels)
  *   TOTEM_TX_GRIDDING  gridding along y onto a twice-finer axis and FFTs (a non-uniform FFT), the
  *                      x phases direct: O(atoms x width + pixels log pixels), relative error
  *                      ~1e-7; used where the axes are uniform and the grid has at most 4096
  *                      rows and 2^30 points, otherwise DIRECT is used.
  * ``scratch_bytes`` bounds the gridding work memory taken during a build (0 = 1 GiB; a quarter of it
- * for each request of a server).  Beyond the bound if need be, a build always takes 48 bytes per atom
- * and 9 n bytes per species of a slice, and the arrays of one species of one slice: at most 64 bytes
- * per pixel of an n x m grid (half of that where both axes are centred on zero), where n is its height
- * rounded up to an edge of the fused transforms and m its width rounded up to 16. */
+ * for each request of a server; less where the device has less).  Beyond the bound if need be, a build
+ * always takes 48 bytes per atom and 9 n bytes per species of a slice, and the arrays of one species of
+ * one slice: at most 64 bytes per pixel of an n x m grid (half of that where both axes are centred on
+ * zero), where n is its height rounded up to an edge of the fused transforms and m its width rounded
+ * up to 16. */
 #define TOTEM_TX_AUTO 0
 #define TOTEM_TX_DIRECT 1
 #define TOTEM_TX_GRIDDING 2

@@ -54,3 +54,38 @@ def test_memory_does_not_grow_with_a_kilobyte_per_atom(engine_lib):
     # 48 bytes an atom of the two species, 64 a pixel and the transmission itself; 64 MB for what the
     # driver keeps (a kilobyte an atom were 205 MB)
     assert taken < 2 * atoms * 48 + 64 * 64 * 72 + (64 << 20), taken
+
+
+def _run(req, mode, scratch, fail=None):
+    with capi.tx_builder(mode, scratch):
+        s = capi.Session(device=0)
+        s.upload(req, stem=False)
+        try:
+            if fail is not None:
+                capi.inject_failures(alloc_after=fail)
+            s.run(what=1)
+        finally:
+            capi.inject_failures()
+        out = s.download(want_transmission=True)[2], s.timing().tx_builder
+        s.close()
+    return out
+
+
+# the build's first allocation is the transmission stack, its second the work memory
+def test_no_room_for_all_slices_takes_them_one_by_one(engine_lib):
+    req = _sparse(_request(64, 512, 3000, slices=3), 50.0 / 3000)
+    want, builder = _run(req, capi.TX_AUTO, 0)
+    assert builder == capi.TX_GRIDDING
+    for mode in (capi.TX_AUTO, capi.TX_GRIDDING):
+        got, builder = _run(req, mode, 0, fail=1)
+        assert builder == capi.TX_GRIDDING and np.array_equal(got, want)
+
+
+def test_no_room_at_all_takes_the_direct_sums_unless_gridding_was_asked_for(engine_lib):
+    req = _sparse(_request(64, 512, 3000, slices=3), 50.0 / 3000)
+    direct, _ = _run(req, capi.TX_DIRECT, 0)
+    got, builder = _run(req, capi.TX_AUTO, 1, fail=1)  # already the least the build can do with
+    assert builder == capi.TX_DIRECT and np.array_equal(got, direct)
+    with pytest.raises(capi.TotemError) as e:
+        _run(req, capi.TX_GRIDDING, 1, fail=1)
+    assert e.value.code == capi.ERR_OOM

@@ -506,8 +506,9 @@ Status totem_session::build_transmission(int path, int* launches) {
     size_t bytes = 0;
     int ex_rows = grid_kmax;
     if (gridding) {
-      // jobs per batch from the budget for their work memory, at least one; a device that has no
-      // room for it takes the direct sums, unless gridding was asked for
+      // jobs per batch from the budget for their work memory, at least one.  A device that has no room
+      // even for a slice's takes the direct sums, unless gridding was asked for: the sums need none, and
+      // grids that always took them must not fail for it (TotemTiming.tx_builder says which ran)
       const int all = grid_job_beg_h.back();
       size_t jobs = std::max(all, 1), per_slice = 1;
       for (int k = 0; k < slices; ++k)
@@ -524,11 +525,23 @@ Status totem_session::build_transmission(int path, int* launches) {
       // a slice needs it, so that a request is split as it is alone (and rounds the same)
       const size_t whole = std::max(limit, need.tables + need.per_job) - need.tables;
       if (grid_scratch.pool) jobs = std::min(jobs, std::max(whole / 4 / need.per_job, per_slice));
-      bytes = need.tables + need.per_job * std::min(whole / need.per_job, jobs);
-      const Status st = grid_scratch.ensure(bytes);
+      jobs = std::min(whole / need.per_job, jobs);
+      bytes = need.tables + need.per_job * jobs;
+      Status st = grid_scratch.ensure(bytes);
+      if (st.code == TOTEM_ERR_OOM) {  // no room: slice by slice and in the smallest pieces, which changes no bit
+        cudaGetLastError();            // (the failed allocation's error)
+        const int least = totem::grid_piece_rows(p_h, p_w, grid_half, grid_kmax, 0);
+        need = totem::grid_bytes(p_h, p_w, grid_half, grid_kmax, least, all, grid_atoms);
+        const size_t small = need.tables + need.per_job * std::min(jobs, per_slice);
+        if (small < bytes) {
+          st = grid_scratch.ensure(small);
+          bytes = small;
+          ex_rows = least;
+        }
+      }
       if (!st.ok()) {
         if (mode == TOTEM_TX_GRIDDING || st.code != TOTEM_ERR_OOM) return st;
-        cudaGetLastError();  // the failed allocation's error
+        cudaGetLastError();
         gridding = false;
       }
     }
