@@ -21,10 +21,13 @@ def _sparse(req, occupancy):
 
 
 @pytest.mark.parametrize("p_h,p_w,atoms,kw", [
-    (64, 64, 1500, {}),                                      # six pieces of 256 groups
+    (64, 64, 1500, {}),
     (64, 30, 700, {"centred": False}),                       # a pitch below 128 columns
-    (64, 512, 3000, {}),                                     # three pieces of columns by six of groups
+    (64, 512, 3000, {}),                                     # phases in pieces of columns
     (96, 96, 5000, {"equal_y": True, "flag": "l"}),          # groups of eight atoms
+    (64, 64, 50_000, {}),                                    # three pieces of groups
+    (64, 512, 20_000, {"centred": False}),                   # four pieces of columns by three of groups
+    (96, 96, 40_000, {"equal_y": True, "flag": "l"}),        # 5000 groups: the last pieces hold none
     (62, 200, 2000, {"centred": False}),
 ])
 def test_phases_in_pieces_change_no_bit(engine_lib, p_h, p_w, atoms, kw):
@@ -51,8 +54,8 @@ def test_memory_does_not_grow_with_a_kilobyte_per_atom(engine_lib):
         s.download()
         taken = free - torch.cuda.mem_get_info()[0]
         s.close()
-    # 48 bytes an atom of the two species, 64 a pixel and the transmission itself; 64 MB for what the
-    # driver keeps (a kilobyte an atom were 205 MB)
+    # tables of the atoms of two species, arrays of the grid, the transmission itself, and 64 MB for the
+    # phases and what the driver keeps (a kilobyte an atom were 205 MB)
     assert taken < 2 * atoms * 48 + 64 * 64 * 72 + (64 << 20), taken
 
 

@@ -662,7 +662,7 @@ GridBytes grid_bytes(int p_h, int p_w, int half, int kmax, int ex_rows, int jobs
 int grid_piece_rows(int p_h, int p_w, int half, int kmax, size_t job_bytes) {
   const size_t rest = grid_bytes(p_h, p_w, half, kmax, 0, 1, 0).per_job;
   const int pitch = (int)grid_pitch(p_w, half), cols = grid_ex_cols(p_h, pitch, kmax);
-  const long long least = std::max(64LL, 4LL * p_h * pitch / cols);
+  const long long least = std::max(4LL * p_h * pitch, 1LL << 20) / cols;
   const long long room = job_bytes > rest ? (long long)((job_bytes - rest) / (cols * sizeof(float2))) : 0;
   return (int)std::min<long long>(kmax, std::max(least, room));
 }
