@@ -207,9 +207,9 @@ TOTEM_API int totem_transmission_run(const TotemStemArgs *args, TotemStemOut *ou
  *                      rows and 2^30 points, otherwise DIRECT is used.
  * ``scratch_bytes`` bounds the gridding work memory taken during a build (0 = 1 GiB; a quarter of it
  * for each request of a server; less where the device has less).  Beyond the bound if need be, a build
- * always takes 48 bytes per atom and 9 n bytes per species of a slice, and the arrays of one species of
- * one slice: at most 64 bytes per pixel of an n x m grid (half of that where both axes are centred on
- * zero), or 8 MB and 32 bytes per pixel, where n is its height rounded up to an edge of the fused
+ * always takes 80 bytes per atom and 9 n bytes per species of a slice, and the arrays of one species of
+ * one slice: at most 96 bytes per pixel of an n x m grid (half of that where both axes are centred on
+ * zero), or 8 MB and 64 bytes per pixel, where n is its height rounded up to an edge of the fused
  * transforms and m its width rounded up to 16. */
 #define TOTEM_TX_AUTO 0
 #define TOTEM_TX_DIRECT 1

@@ -152,7 +152,7 @@ struct GridWork {
   int kmax = 0;                    // atoms of the largest job
   int cols = 0, pitch = 0, half = 0;  // columns formed (p_w, or p_w / 2 + 1 when half), row pitch
   // all jobs; a job's atoms start at GridPlanDev::atom_beg
-  float4* wgt = nullptr;           // [atoms][2]: the spreading weights of every group
+  double* wgt = nullptr;           // [atoms][8]: the spreading weights of every group
   int* bin = nullptr;              // [atoms]: first fine row of every atom (job order)
   int* base = nullptr;             // [atoms]: first fine row of every group
   int* order = nullptr;            // [atoms]: the job's atoms sorted by fine row
@@ -165,6 +165,7 @@ struct GridWork {
   int ex_rows = 0;                 // groups of E held at a time (kmax, or fewer)
   float2* ex = nullptr;            // [jobs][ex_rows][ex_cols]
   float2* fine = nullptr;          // [jobs][2 n][pitch]
+  double2* fine64 = nullptr;       // the same rows between two pieces of the groups (ex_rows < kmax)
   float2* s = nullptr;             // [jobs][p_h + 1][pitch]
 };
 struct GridBatch {
@@ -179,7 +180,7 @@ struct GridBytes {
 GridBytes grid_bytes(int p_h, int p_w, int half, int kmax, int ex_rows, int jobs, long long atoms);
 // ex_rows for which a job's large arrays take ``job_bytes``; not above kmax, and not below what makes the
 // phases 4 p_h rows or 8 MB large (with less, too few groups are at hand to fill the device: 10 000 atoms
-// on 256^2 in pieces of 1.2 MB 23.8 ms, of 8 MB 12.4 ms).
+// on 256^2 in pieces of 1.2 MB 39.7 ms, of 8 MB 10.7 ms).
 int grid_piece_rows(int p_h, int p_w, int half, int kmax, size_t job_bytes);
 // Overwrites out like launch_tx_species; ``scratch`` holds the tables and at least one job's arrays.
 // With ``finish`` (the transmission's fused FFT takes the grid and nothing is to be added to V) out

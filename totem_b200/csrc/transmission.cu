@@ -386,7 +386,14 @@ __global__ void __launch_bounds__(GR_T) k_grid_sort(GridPlanDev gp, SpeciesSet s
   }
 }
 
-// E[group][column]: the direct x phases, summed over the group's atoms, and the groups' spreading
+// exp(-2 pi i t) for t given in FP64, reduced to [-1/2, 1/2]: half the rounding of phase_of's [0, 1).
+__device__ __forceinline__ float2 near_phase_of(double t) {
+  float s, c;
+  sincospif(2.f * (float)(t - rint(t)), &s, &c);
+  return make_float2(c, -s);
+}
+
+// E[group][column]: the direct x phases, summed over the group's atoms in FP64, and the groups' spreading
 // weights, for the groups [g0, g0 + ex_rows).  A CTA takes 128 columns of every gridDim.y-th chunk of 16
 // groups of one job.
 __global__ void __launch_bounds__(128) k_grid_phases(GridPlanDev gp, SpeciesSet spset, TxGrid g, int job0,
@@ -396,7 +403,7 @@ __global__ void __launch_bounds__(128) k_grid_phases(GridPlanDev gp, SpeciesSet 
   const double* pos = spset.k[jb.x & 3].pos + 2L * jb.z;
   const int* order = w.order + gp.atom_beg[job];
   const int* first = w.first + gp.atom_beg[job] + job;
-  float* wgt = reinterpret_cast<float*>(w.wgt + 2L * gp.atom_beg[job]);
+  double* wgt = w.wgt + (long)GR_W * gp.atom_beg[job];
   float2* ex = w.ex + (long)blockIdx.z * w.ex_rows * w.ex_cols + (h - col0);
   const int groups = min(w.groups[job], g0 + w.ex_rows);
   // half: column h holds kx = h dkx, the last of them +p_w / 2 (the grid's own -p_w / 2 is its
@@ -411,80 +418,118 @@ __global__ void __launch_bounds__(128) k_grid_phases(GridPlanDev gp, SpeciesSet 
       if (q < groups) {
         const double v = fine_row(pos[2L * order[first[q]] + 1], gp.dky, 2 * gp.n);
         const double d = (ceil(v - GR_W / 2) + k - v) / (GR_W / 2);
-        wgt[GR_W * q + k] = (float)(bessel_i0(GR_BETA * sqrt(fmax(1.0 - d * d, 0.0))) * (1.0 / bessel_i0(GR_BETA)));
+        wgt[GR_W * q + k] = bessel_i0(GR_BETA * sqrt(fmax(1.0 - d * d, 0.0))) * (1.0 / bessel_i0(GR_BETA));
       }
     }
     if (h >= w.pitch) continue;
     for (int q = q0; q < min(q0 + 16, groups); ++q) {
-      float2 s = make_float2(0.f, 0.f);
+      double2 s = make_double2(0.0, 0.0);
       for (int i = first[q]; i < first[q + 1]; ++i) {
         const double* p = pos + 2L * order[i];
-        s = cadd(s, phase_of(kx * p[0] + (w.half ? 0.0 : gp.sy * p[1])));
+        const float2 e = near_phase_of(kx * p[0] + (w.half ? 0.0 : gp.sy * p[1]));
+        s = make_double2(s.x + e.x, s.y + e.y);
       }
-      ex[(long)(q - g0) * w.ex_cols] = s;
+      ex[(long)(q - g0) * w.ex_cols] = make_float2((float)s.x, (float)s.y);
     }
   }
 }
 
 // Adds weight times x of a group whose first fine row lies D rows from the block's.
 template <int D>
-__device__ __forceinline__ void spread_at(float2 (&acc)[GR_ROWS], const float* wt, float2 x) {
+__device__ __forceinline__ void spread_at(double2 (&acc)[GR_ROWS], const double* wt, double2 x) {
 #pragma unroll
   for (int k = 0; k < GR_W; ++k)
-    if (D + k >= 0 && D + k < GR_ROWS) acc[D + k] = __ffma2_rn(make_float2(wt[k], wt[k]), x, acc[D + k]);
+    if (D + k >= 0 && D + k < GR_ROWS)
+      acc[D + k] = make_double2(fma(wt[k], x.x, acc[D + k].x), fma(wt[k], x.y, acc[D + k].y));
 }
 
 // One block of GR_ROWS fine rows of one job and 128 columns, a column per thread: the groups that
 // reach the block in sorted order.  All lanes take the same group, so its offset picks one of the 23
-// unrolled bodies without divergence and the weights are uniform loads; E is loaded four groups
-// ahead of its use.  PIECES: of the groups only [g0, g0 + ex_rows) are held: from the second such piece on the
-// sums continue from the rows in memory, in the same order (the groups that wrap around sort last), so
-// the pieces change no bit.
+// unrolled bodies without divergence; the weights and rows of the next 16 groups are staged in shared
+// memory while the present ones are added, and E is loaded four groups ahead of its use.
+// The sums are FP64 and rounded once, whatever the atoms per row (25 000 terms on a row of 64^2: the
+// transmission 1.3e-7 from 64 bits, with FP32 sums 2.0e-5; on grids filled with SrTiO3 it was 0.1-0.9 %
+// further off with FP32 sums and phases reduced to [0, 1)). 64 instead of 32 registers of sums and half the FMA rate cost 27 us
+// on 66 at 2048^2 with 10 jobs of 1024 atoms, 4.6 % of a build.  Slower still: weights read from global
+// memory by every thread (+20 us), a thread per real component, half the registers and twice the
+// threads (+42 us), E loaded eight groups ahead (126 registers, +12 us).
+// PIECES: of the groups only [g0, g0 + ex_rows) are held.  The sums go on from one piece to the next in
+// fine64, in the same order (the groups that wrap around sort last), so the pieces change no bit.
 template <bool PIECES>
 __global__ void __launch_bounds__(128) k_grid_spread(GridPlanDev gp, int job0, int col0, int g0, GridWork w) {
   const int nf = 2 * gp.n, f0 = blockIdx.y * GR_ROWS, job = job0 + blockIdx.z;
   const int h = col0 + blockIdx.x * 128 + threadIdx.x;
   if (!w.used[(long)job * (nf / GR_ROWS) + blockIdx.y]) return;
+  constexpr int GR_Q = 128 / GR_W;  // groups whose weights and rows are staged at a time
+  __shared__ double s_w[GR_Q][GR_W];
+  __shared__ int s_row[GR_Q];
   const int hc = min(h, w.pitch - 1);
   const int* __restrict__ ptr = w.ptr + (long)job * (nf + 1);
   const int* __restrict__ base = w.base + gp.atom_beg[job];
-  const float4* __restrict__ wgt = w.wgt + 2L * gp.atom_beg[job];
+  const double* __restrict__ wgt = w.wgt + (long)GR_W * gp.atom_beg[job];
   const float2* __restrict__ ex = w.ex + ((long)blockIdx.z * w.ex_rows - (PIECES ? g0 : 0)) * w.ex_cols + (hc - col0);
-  float2* dst = w.fine + ((long)blockIdx.z * nf + f0) * w.pitch + hc;
-  float2 acc[GR_ROWS];
+  const long at = ((long)blockIdx.z * nf + f0) * w.pitch + hc;
+  // the groups of the block, and those that wrap around into the first one
+  int lo = ptr[max(f0 - GR_W + 1, 0)], hi = ptr[f0 + GR_ROWS];
+  int wlo = f0 == 0 ? ptr[nf - GR_W + 1] : 0, whi = f0 == 0 ? ptr[nf] : 0;
+  const bool last = !PIECES || g0 + w.ex_rows >= w.kmax;
+  if (PIECES) {
+    lo = max(lo, g0), hi = min(hi, g0 + w.ex_rows);
+    wlo = max(wlo, g0), whi = min(whi, g0 + w.ex_rows);
+    if (g0 > 0 && !last && lo >= hi && wlo >= whi) return;
+  }
+  double2 acc[GR_ROWS];
 #pragma unroll
-  for (int t = 0; t < GR_ROWS; ++t) acc[t] = PIECES && g0 > 0 ? dst[(long)t * w.pitch] : make_float2(0.f, 0.f);
-  for (int wrap = 0; wrap <= (f0 == 0 ? 1 : 0); ++wrap) {
-    int lo = ptr[wrap ? nf - GR_W + 1 : max(f0 - GR_W + 1, 0)], hi = ptr[wrap ? nf : f0 + GR_ROWS];
-    if (PIECES) {
-      lo = max(lo, g0);
-      hi = min(hi, g0 + w.ex_rows);
-    }
+  for (int t = 0; t < GR_ROWS; ++t)
+    acc[t] = PIECES && g0 > 0 ? w.fine64[at + (long)t * w.pitch] : make_double2(0.0, 0.0);
+  const int tq = threadIdx.x / GR_W, tk = threadIdx.x % GR_W;
+  for (int wrap = 0; wrap < 2; ++wrap, lo = wlo, hi = whi) {
     const int shift = (wrap ? nf : 0) + f0;
-    for (int q0 = lo; q0 < hi; q0 += 4) {
-      float2 x[4];
+    double next_w = 0.0;
+    int next_row = 0;
+    if (lo + tq < hi) {
+      next_w = __ldg(wgt + (long)GR_W * (lo + tq) + tk);
+      next_row = __ldg(base + lo + tq);
+    }
+    for (int q0 = lo; q0 < hi; q0 += GR_Q) {
+      __syncthreads();  // the previous groups' weights are read
+      s_w[tq][tk] = next_w;
+      if (tk == 0) s_row[tq] = next_row - shift;
+      __syncthreads();
+      if (q0 + GR_Q + tq < hi) {
+        next_w = __ldg(wgt + (long)GR_W * (q0 + GR_Q + tq) + tk);
+        next_row = __ldg(base + q0 + GR_Q + tq);
+      }
+      const int m = min(GR_Q, hi - q0);
+      for (int i0 = 0; i0 < m; i0 += 4) {
+        float2 x[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) x[i] = q0 + i < hi ? __ldg(ex + (long)(q0 + i) * w.ex_cols) : make_float2(0.f, 0.f);
+        for (int i = 0; i < 4; ++i)
+          x[i] = i0 + i < m ? __ldg(ex + (long)(q0 + i0 + i) * w.ex_cols) : make_float2(0.f, 0.f);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (q0 + i >= hi) break;
-        const float4 wa = __ldg(wgt + 2 * (q0 + i)), wb = __ldg(wgt + 2 * (q0 + i) + 1);
-        const float wt[GR_W] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
-        switch (__ldg(base + q0 + i) - shift) {
+        for (int i = 0; i < 4; ++i) {
+          if (i0 + i >= m) break;
+          const double2 xi = make_double2(x[i].x, x[i].y);
+          const double* wt = s_w[i0 + i];
+          switch (s_row[i0 + i]) {
 #define TOTEM_SPREAD(D) \
-  case D: spread_at<D>(acc, wt, x[i]); break;
-          TOTEM_SPREAD(-7) TOTEM_SPREAD(-6) TOTEM_SPREAD(-5) TOTEM_SPREAD(-4) TOTEM_SPREAD(-3) TOTEM_SPREAD(-2)
-          TOTEM_SPREAD(-1) TOTEM_SPREAD(0) TOTEM_SPREAD(1) TOTEM_SPREAD(2) TOTEM_SPREAD(3) TOTEM_SPREAD(4)
-          TOTEM_SPREAD(5) TOTEM_SPREAD(6) TOTEM_SPREAD(7) TOTEM_SPREAD(8) TOTEM_SPREAD(9) TOTEM_SPREAD(10)
-          TOTEM_SPREAD(11) TOTEM_SPREAD(12) TOTEM_SPREAD(13) TOTEM_SPREAD(14) TOTEM_SPREAD(15)
+  case D: spread_at<D>(acc, wt, xi); break;
+            TOTEM_SPREAD(-7) TOTEM_SPREAD(-6) TOTEM_SPREAD(-5) TOTEM_SPREAD(-4) TOTEM_SPREAD(-3) TOTEM_SPREAD(-2)
+            TOTEM_SPREAD(-1) TOTEM_SPREAD(0) TOTEM_SPREAD(1) TOTEM_SPREAD(2) TOTEM_SPREAD(3) TOTEM_SPREAD(4)
+            TOTEM_SPREAD(5) TOTEM_SPREAD(6) TOTEM_SPREAD(7) TOTEM_SPREAD(8) TOTEM_SPREAD(9) TOTEM_SPREAD(10)
+            TOTEM_SPREAD(11) TOTEM_SPREAD(12) TOTEM_SPREAD(13) TOTEM_SPREAD(14) TOTEM_SPREAD(15)
 #undef TOTEM_SPREAD
+          }
         }
       }
     }
   }
   if (h >= w.pitch) return;
 #pragma unroll
-  for (int t = 0; t < GR_ROWS; ++t) dst[(long)t * w.pitch] = acc[t];
+  for (int t = 0; t < GR_ROWS; ++t) {
+    if (last) w.fine[at + (long)t * w.pitch] = make_float2((float)acc[t].x, (float)acc[t].y);
+    else w.fine64[at + (long)t * w.pitch] = acc[t];
+  }
 }
 
 // V(r, c) of slices s_lo.. from the jobs [j_lo, j_hi): f_species(s^2) S summed over the jobs,
@@ -541,7 +586,7 @@ size_t grid_work(int p_h, int p_w, int half, int kmax, int ex_rows, int jobs, lo
     return p;
   };
   const size_t nj = jobs, na = (size_t)atoms, nb = batch, row = w->pitch * sizeof(float2);
-  w->wgt = reinterpret_cast<float4*>(take(na * 2 * sizeof(float4)));
+  w->wgt = reinterpret_cast<double*>(take(na * GR_W * sizeof(double)));
   w->bin = reinterpret_cast<int*>(take(na * sizeof(int)));
   w->base = reinterpret_cast<int*>(take(na * sizeof(int)));
   w->order = reinterpret_cast<int*>(take(na * sizeof(int)));
@@ -555,6 +600,7 @@ size_t grid_work(int p_h, int p_w, int half, int kmax, int ex_rows, int jobs, lo
   w->ex = reinterpret_cast<float2*>(take(nb * w->ex_rows * w->ex_cols * sizeof(float2)));
   w->fine = reinterpret_cast<float2*>(take(nb * 2 * n * row));
   w->s = reinterpret_cast<float2*>(take(nb * (p_h + 1) * row));
+  w->fine64 = reinterpret_cast<double2*>(take(ex_rows < kmax ? nb * 2 * n * w->pitch * sizeof(double2) : 0));
   return off;
 }
 

@@ -26,7 +26,7 @@
 // oversampling 2 and beta = pi sqrt((W/2)^2 (3/2)^2 - 0.8) (Beatty, Nishimura & Pauly, IEEE Trans.
 // Med. Imaging 24 (2005) 799-808), whose transform W sinh(z)/(z I0(beta)), z = sqrt(beta^2 -
 // (pi W xi)^2), is divided out.  The aliasing error is ~2e-8 of S at the largest |ky| and less
-// below, under the FP32 rounding of the sums.
+// below, under the FP32 rounding of the transforms; the weights and the fine rows' sums are FP64.
 //
 // Why this split: a 2-D fine grid (2P x 2P points per job) was 64 bytes per pixel and job of clearing,
 // spreading, row and column passes: 29-44 ps per pixel and job.  With the x factor direct, nothing
