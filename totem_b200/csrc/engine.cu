@@ -805,16 +805,36 @@ Status totem_session::slice_loop(int path, int batch, bool batch_fixed, int col_
   }
   auto tslice = [&](int k) { return static_cast<const char*>(Tslices) + (size_t)k * tslice_bytes; };
 
-  auto enqueue_batches = [&]() -> Status {
-    int turn = 0;
-    for (long item0 = 0; item0 < items_total; item0 += B, turn = (turn + 1) % chains) {
-      const cudaStream_t st = turn == 0 ? stream : stream2;
-      double* part_e = part.as<double>() + turn * n_events * part_stride;
-      const int items = (int)std::min<long>(B, items_total - item0);
-      if (fused) {
-        totem::SliceLoopArgs s;
-        s.n = h; s.items = items; s.item0 = (int)item0; s.geo = geo; s.p_h = p_h;
-        s.psi = psi.as<float2>() + turn * (size_t)B * vol; s.probe = probe.as<float2>(); s.prop = prop.as<float2>();
+  // detector sums of one batch, whose partial sums start at part_e
+  auto reduce = [&](double* part_e, int items, long item0, cudaStream_t st) -> Status {
+    for (int e = 0; e < n_events; ++e) {
+      TOTEM_TRY(totem::launch_det_reduce(part_e + e * part_stride, nblk, aper_num, items, (int)item0, depth,
+                                         acc.as<double>() + (size_t)e * w_num * ad, st, skip));
+      ++*launches;
+    }
+    return Status::Ok();
+  };
+
+  // One batch, or two side by side: their passes are enqueued in turn, so that the second chain starts
+  // with the first instead of after all its launches (20 slices of 1024^2 without a graph: 82 launches
+  // of 10 us and more, one chain alone for as long as the host takes to enqueue them).
+  auto enqueue_fused = [&]() -> Status {
+    struct Batch {
+      totem::SliceLoopArgs s;
+      double* part_e;
+      cudaStream_t st;
+    };
+    for (long first = 0; first < items_total; first += (long)chains * B) {
+      Batch batch[2];
+      int nb = 0;
+      for (; nb < chains && first + (long)nb * B < items_total; ++nb) {
+        Batch& b = batch[nb];
+        const long item0 = first + (long)nb * B;
+        b.st = nb == 0 ? stream : stream2;
+        b.part_e = part.as<double>() + nb * n_events * part_stride;
+        totem::SliceLoopArgs& s = b.s;
+        s.n = h; s.items = (int)std::min<long>(B, items_total - item0); s.item0 = (int)item0; s.geo = geo; s.p_h = p_h;
+        s.psi = psi.as<float2>() + nb * (size_t)B * vol; s.probe = probe.as<float2>(); s.prop = prop.as<float2>();
         s.tw = tw_n.as<float2>(); s.aper_num = aper_num;
         s.mask_mid = mask_mid.as<float>(); s.mask_exit = mask_exit.as<float>();
         s.col_variant = col_variant;
@@ -823,70 +843,71 @@ Status totem_session::slice_loop(int path, int batch, bool batch_fixed, int col_
         s.skip_rows = skip_rows ? 1 : 0;
         s.row_variant = row_variant;
         s.overlap = (chains == 1 && !profiling && overlap_pays(h)) ? 1 : 0;
-        TOTEM_TRY(prof_begin());
-        TOTEM_TRY(totem::launch_row_pass(s, tslice(0), true, st));
-        TOTEM_TRY(prof_end(0));
-        ++*launches;
-        for (int k = 0; k < slices; ++k) {
-          const int ev_mid = event_of_slice[k + 1];
-          int flags = 0;
-          if (ev_mid >= 0) {
-            flags |= 1;
-            s.part_mid = part_e + ev_mid * part_stride;
-          }
-          if (k == slices - 1) {
-            flags |= 2 | 4;
-            s.part_exit = part_e + exit_event * part_stride;
-          }
+      }
+      auto row_passes = [&](int k) -> Status {
+        for (int i = 0; i < nb; ++i) {
           TOTEM_TRY(prof_begin());
-          TOTEM_TRY(totem::launch_col_pass(s, flags, st));
+          TOTEM_TRY(totem::launch_row_pass(batch[i].s, tslice(k), k == 0, batch[i].st));
+          TOTEM_TRY(prof_end(0));
+          ++*launches;
+        }
+        return Status::Ok();
+      };
+      TOTEM_TRY(row_passes(0));
+      for (int k = 0; k < slices; ++k) {
+        const int ev_mid = event_of_slice[k + 1];
+        const int flags = (ev_mid >= 0 ? 1 : 0) | (k == slices - 1 ? 2 | 4 : 0);
+        for (int i = 0; i < nb; ++i) {
+          if (ev_mid >= 0) batch[i].s.part_mid = batch[i].part_e + ev_mid * part_stride;
+          if (k == slices - 1) batch[i].s.part_exit = batch[i].part_e + exit_event * part_stride;
+          TOTEM_TRY(prof_begin());
+          TOTEM_TRY(totem::launch_col_pass(batch[i].s, flags, batch[i].st));
           TOTEM_TRY(prof_end(1));
           ++*launches;
-          if (k < slices - 1) {
-            TOTEM_TRY(prof_begin());
-            TOTEM_TRY(totem::launch_row_pass(s, tslice(k + 1), false, st));
-            TOTEM_TRY(prof_end(0));
-            ++*launches;
-          }
         }
-      } else {
-        cufftHandle p;
-        TOTEM_TRY(plan(h, w, items, &p));
-        float2* ps = psi.as<float2>();
-        for (int k = 0; k < slices; ++k) {
-          // the probe enters with the first slice's T, the last IFFT's 1 / N^2 with each later one's
-          TOTEM_TRY(totem::launch_plain_gather_mul(ps, k == 0 ? probe.as<float2>() : nullptr, Tp + (size_t)k * plane, h,
-                                                   w, items, (int)item0, geo, k == 0 ? 1.f : 1.f / (float)vol, stream));
-          TOTEM_CUFFT(cufftExecC2C(p, (cufftComplex*)ps, (cufftComplex*)ps, CUFFT_FORWARD));
-          TOTEM_TRY(totem::launch_plain_mul(ps, prop.as<float2>(), (int)vol, items, stream));
-          *launches += 3;
-          const int ev_mid = event_of_slice[k + 1];
-          if (ev_mid >= 0) {
-            TOTEM_TRY(totem::launch_plain_detect(ps, mask_mid.as<float>(), aper_num, (int)vol, items,
-                                                 part_e + ev_mid * part_stride, nblk, stream));
-            ++*launches;
-          }
-          // the exit detectors' FFT cancels the last slice's IFFT: they take its spectrum
-          if (k < slices - 1) {
-            TOTEM_CUFFT(cufftExecC2C(p, (cufftComplex*)ps, (cufftComplex*)ps, CUFFT_INVERSE));
-            ++*launches;
-          }
-        }
-        if (slices == 0) {  // no specimen: the probes' own spectra
-          TOTEM_TRY(totem::launch_plain_gather_mul(ps, probe.as<float2>(), nullptr, h, w, items, (int)item0, geo, 1.f,
-                                                   stream));
-          TOTEM_CUFFT(cufftExecC2C(p, (cufftComplex*)ps, (cufftComplex*)ps, CUFFT_FORWARD));
-          *launches += 2;
-        }
-        TOTEM_TRY(totem::launch_plain_detect(ps, mask_exit.as<float>(), aper_num, (int)vol, items,
-                                             part_e + exit_event * part_stride, nblk, stream));
-        ++*launches;
+        if (k < slices - 1) TOTEM_TRY(row_passes(k + 1));
       }
-      for (int e = 0; e < n_events; ++e) {
-        TOTEM_TRY(totem::launch_det_reduce(part_e + e * part_stride, nblk, aper_num, items, (int)item0, depth,
-                                           acc.as<double>() + (size_t)e * w_num * ad, st, skip));
-        ++*launches;
+      for (int i = 0; i < nb; ++i) TOTEM_TRY(reduce(batch[i].part_e, batch[i].s.items, batch[i].s.item0, batch[i].st));
+    }
+    return Status::Ok();
+  };
+
+  auto enqueue_plain = [&]() -> Status {
+    double* part_e = part.as<double>();
+    for (long item0 = 0; item0 < items_total; item0 += B) {
+      const int items = (int)std::min<long>(B, items_total - item0);
+      cufftHandle p;
+      TOTEM_TRY(plan(h, w, items, &p));
+      float2* ps = psi.as<float2>();
+      for (int k = 0; k < slices; ++k) {
+        // the probe enters with the first slice's T, the last IFFT's 1 / N^2 with each later one's
+        TOTEM_TRY(totem::launch_plain_gather_mul(ps, k == 0 ? probe.as<float2>() : nullptr, Tp + (size_t)k * plane, h,
+                                                 w, items, (int)item0, geo, k == 0 ? 1.f : 1.f / (float)vol, stream));
+        TOTEM_CUFFT(cufftExecC2C(p, (cufftComplex*)ps, (cufftComplex*)ps, CUFFT_FORWARD));
+        TOTEM_TRY(totem::launch_plain_mul(ps, prop.as<float2>(), (int)vol, items, stream));
+        *launches += 3;
+        const int ev_mid = event_of_slice[k + 1];
+        if (ev_mid >= 0) {
+          TOTEM_TRY(totem::launch_plain_detect(ps, mask_mid.as<float>(), aper_num, (int)vol, items,
+                                               part_e + ev_mid * part_stride, nblk, stream));
+          ++*launches;
+        }
+        // the exit detectors' FFT cancels the last slice's IFFT: they take its spectrum
+        if (k < slices - 1) {
+          TOTEM_CUFFT(cufftExecC2C(p, (cufftComplex*)ps, (cufftComplex*)ps, CUFFT_INVERSE));
+          ++*launches;
+        }
       }
+      if (slices == 0) {  // no specimen: the probes' own spectra
+        TOTEM_TRY(totem::launch_plain_gather_mul(ps, probe.as<float2>(), nullptr, h, w, items, (int)item0, geo, 1.f,
+                                                 stream));
+        TOTEM_CUFFT(cufftExecC2C(p, (cufftComplex*)ps, (cufftComplex*)ps, CUFFT_FORWARD));
+        *launches += 2;
+      }
+      TOTEM_TRY(totem::launch_plain_detect(ps, mask_exit.as<float>(), aper_num, (int)vol, items,
+                                           part_e + exit_event * part_stride, nblk, stream));
+      ++*launches;
+      TOTEM_TRY(reduce(part_e, items, item0, stream));
     }
     return Status::Ok();
   };
@@ -900,7 +921,7 @@ Status totem_session::slice_loop(int path, int batch, bool batch_fixed, int col_
       TOTEM_CUDA(cudaEventRecord(fork_ev, stream));
       TOTEM_CUDA(cudaStreamWaitEvent(stream2, fork_ev, 0));
     }
-    const Status st = enqueue_batches();
+    const Status st = fused ? enqueue_fused() : enqueue_plain();
     if (chains > 1) {  // joined whether or not every launch succeeded: nothing outlives the run
       TOTEM_CUDA(cudaEventRecord(join_ev, stream2));
       TOTEM_CUDA(cudaStreamWaitEvent(stream, join_ev, 0));
