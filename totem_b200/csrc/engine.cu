@@ -697,8 +697,12 @@ namespace {
 //  * Waves of both chains together: 50 MB up to 576^2, 32 MB above (512^2 at 32 / 44 / 56 / 68 MB:
 //    1.291 / 1.253 / 1.247 / 1.253; 640^2 3.662 / 3.716 / 3.904 / 4.071).  Windows of which L2 does
 //    not hold two (2048^2) still gain from the overlap; eight a batch was best.
-//  * 1536^2 windows stream faster than they run from L2 (21.86 against 22.70 us; a launch over one
-//    or two of them is barely a wave of CTAs): one batch, once there are enough to amortise it.
+//  * 1536^2 windows run 1.5-5 % faster in one batch from 0.35 GB of waves on (20 / 60 / 120 items, one
+//    batch against two chains: 22.73 / 22.14 / 21.98 against 23.07 / 23.09 / 23.21).  No other window
+//    differs by as much: from 1 GB on one batch is 1-2.5 % faster at 640^2 (3.52 / 3.60), 768^2 (4.30 /
+//    4.36), 800^2 (5.98 / 6.07) and 1152^2 (12.90 / 13.20), and within 1 % at 1024^2 and 1280^2; chains stay
+//    faster at 576^2 (2.12 / 2.10), 1600^2 (29.6 / 29.3) and 2048^2, and at nearly every window below
+//    0.2 GB (by 2 to 14 %).
 //  * Below 1.5 M points in all, one launch does not fill the GPU and two only add launches (256^2, 8
 //    items 1.084 / 1.142, 16 items 0.708 / 0.715, 64 items 0.397 / 0.321; 512^2, 4 items 3.22 / 3.34,
 //    8 items 2.39 / 2.25).
@@ -816,8 +820,8 @@ Status totem_session::slice_loop(int path, int batch, bool batch_fixed, int col_
   };
 
   // One batch, or two side by side: their passes are enqueued in turn, so that the second chain starts
-  // with the first instead of after all its launches (20 slices of 1024^2 without a graph: 82 launches
-  // of 10 us and more, one chain alone for as long as the host takes to enqueue them).
+  // with the first instead of after all its launches.  Launched without a graph, one after the other / in
+  // turn: 64 probes of 512^2 over 40 slices 3.29 / 3.14 ms, 400 of 64^2 0.87 / 0.65 ms.
   auto enqueue_fused = [&]() -> Status {
     struct Batch {
       totem::SliceLoopArgs s;
