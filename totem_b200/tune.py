@@ -10,8 +10,9 @@ events around the device work, transmission excluded, best of ``--reps`` runs af
   * the column-pass variants (TotemRunOptions.col_variant: 1 default, 2 propagator in shared
     memory, 3 lower register cap, 5 8-column tiles, 6 32-column tiles where they exist),
   * the row-pass variants (row_variant: 1 default, 3 / 4 / 5 resident 128-thread CTAs per SM),
-  * batches of 1, 2 and 4 GiB of probe waves,
+  * bounds of 1, 2 and 4 GiB on a batch's probe waves, where the engine's plan comes near them,
 
+each as the engine runs it by default (two chains of batches that fit L2, or one streaming batch),
 by coordinate descent (column variant, then row variant, then batch, then the column variant
 once more).  Each size's choice goes into the table as one JSON line; the engine reads it for runs
 that leave those options at 0 (``totem_load_tuning``).  Entries of other GPUs and sizes are kept.
@@ -66,18 +67,22 @@ class Timer:
         self.sess.upload(req)
         self.sess.run(row_variant=1, col_variant=1, batch=1)  # transmission
         self.cache = {}
+        self.planned_mib = 0.0  # waves of a batch of the engine's plan
 
     def __call__(self, rv: int, cv: int, batch_mib: int) -> float:
         key = (rv, cv, batch_mib)
         if key not in self.cache:
             n = self.req.height
-            batch = max(1, (batch_mib << 20) // (n * n * 8))
+            # the largest bound is the engine's own: batch 0 runs its plan; a smaller one is given as a batch
+            batch = 0 if batch_mib == max(BATCH_MIB) else max(1, (batch_mib << 20) // (n * n * 8))
             best = float("inf")
             for i in range(self.reps + 1):
                 self.sess.run(skip_transmission=True, row_variant=rv, col_variant=cv, batch=batch)
                 t = self.sess.timing()
                 if i:  # the first run of a shape is the warm-up (and is captured for graph replay next)
                     best = min(best, t.slice_loop_ms)
+            if batch == 0:
+                self.planned_mib = t.batch * n * n * 8 / 2 ** 20
             self.cache[key] = 1e3 * best / self.req.probe_slices
         return self.cache[key]
 
@@ -96,7 +101,7 @@ def tune_size(n: int, device: int = 0, reps: int = 3, log=print):
                 cv = min(col_variants(n), key=lambda v: tm(rv, v, bm))
             elif stage == "row":
                 rv = min(row_variants(n), key=lambda v: tm(v, cv, bm))
-            else:
+            elif tm.planned_mib > min(BATCH_MIB):  # a plan of smaller batches takes no notice of the bound
                 bm = min(BATCH_MIB, key=lambda b: tm(rv, cv, b))
         best = tm(rv, cv, bm)
         log(f"n={n}: row {rv} col {cv} batch {bm} MiB: {best:.4f} us per probe*slice "
