@@ -102,15 +102,16 @@ size_t resident_bytes(const TotemStemArgs& a) {
 }
 
 // Estimated device time of a request in seconds, for ordering preparation under the SHORTEST
-// policy: slice loop ~7.2 ps per probe-slice pixel, transmission build ~1.6 ps per atom-pixel
-// (SrTiO3 on B200: 1.9 us per probe-slice at 512^2; 27 ms for 16 000 atoms on a 1024^2 grid).
+// policy (B200): slice loop ~4.6 ps per probe-slice pixel (1.19 us per probe-slice at 512^2);
+// transmission build per slice and pixel ~22 ps of transforms and form factors and 0.29 ps per atom
+// by the direct sums, at most the ~36 ps of gridding (3.1 ms for 20 slices of 2048^2).
 double est_seconds(const TotemStemArgs& a) {
   long long atoms = 0;
   for (const double* cnt : {a.atom_slice, a.atom_slice_i})
     if (cnt)
       for (int s = 0; s < a.slices; ++s) atoms += (long long)cnt[s];
-  const double loop = 7.2e-12 * (double)a.w_num * a.depth * a.slices * (double)a.height * a.width;
-  const double tx = 1.6e-12 * (double)atoms * a.p_height * a.p_width;
+  const double loop = 4.6e-12 * (double)a.w_num * a.depth * a.slices * (double)a.height * a.width;
+  const double tx = std::min(22e-12 * a.slices + 0.29e-12 * (double)atoms, 36e-12 * a.slices) * a.p_height * a.p_width;
   return loop + tx;
 }
 
