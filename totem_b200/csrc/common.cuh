@@ -126,9 +126,9 @@ Status launch_tx_structure(const TxGrid& g, const AtomRowsDev& neutral, const At
 // Overwrites out.
 Status launch_tx_species(const TxGrid& g, const SpeciesSet& sp, float2* out, cudaStream_t st);
 // The same sums by gridding along y (tx_grid.cuh) on separable grids with a uniform ky axis, up to
-// 4096 rows.  Work is grouped in jobs, one per (slice, kind, species)
-// segment, ordered by slice; a batch runs the jobs [j_lo, j_hi) in scratch memory and writes slices
-// [s_lo, s_hi) (the last may be partial, finished by the next batch).
+// 4096 rows (and grid_indexes_fit).  Work is grouped in jobs, one per (slice, kind, species) segment,
+// ordered by slice; a batch runs the jobs [j_lo, j_hi) in scratch memory and writes slices [s_lo, s_hi):
+// whole slices, or where a batch does not hold one, parts of a slice that the next batch adds to.
 struct GridPlanDev {
   int n = 0;                       // transform length: grid_transform(p_h)
   double dky = 0;                  // spacing of the ky axis
@@ -387,9 +387,9 @@ Status launch_plain_scale(float2* psi, float s, long total, cudaStream_t st);
 Status launch_plain_tf_mul(float2* work, const float2* spec, const float2* tf, int vol, int planes, cudaStream_t st);
 Status launch_plain_image(const float2* work, int planes, const double* w, float s, int vol, float* out,
                           cudaStream_t st);
-// CBED: out[h][w] = sum_q gfsf[q] |fftshift(spec_q)|^2 over w_num kept spectra [w_num][h][w] (FP64).
 // out[i] = 1 (complex64): the plane incident wave of HRTEM.
 Status launch_fill_ones(float2* out, long n, cudaStream_t st);
+// CBED: out[h][w] = sum_q gfsf[q] |fftshift(spec_q)|^2 over w_num kept spectra [w_num][h][w] (FP64).
 Status launch_cbed_pattern(const float2* spec, const double* gfsf, int w_num, int h, int w, double* out,
                            cudaStream_t st);
 Status launch_plain_detect(const float2* psi, const float* masks, int aper_num, int vol, int items,

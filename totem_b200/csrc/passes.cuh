@@ -1,6 +1,6 @@
 // Kernel templates of the fused slice loop and of continuous batching, instantiated per window
 // size by the files that dispatch on it (power-of-two windows: rowpass.cu, multislice.cu,
-// groups.cu; mixed-radix windows: windows_mixed_*.cu).
+// groups.cu; mixed-radix windows: windows_mr_*.cu).
 #pragma once
 #include "hrtem_kernels.cuh"
 #include "tx_grid.cuh"

@@ -449,10 +449,10 @@ __device__ __forceinline__ void spread_at(double2 (&acc)[GR_ROWS], const double*
 // memory while the present ones are added, and E is loaded four groups ahead of its use.
 // The sums are FP64 and rounded once, whatever the atoms per row (25 000 terms on a row of 64^2: the
 // transmission 1.3e-7 from 64 bits, with FP32 sums 2.0e-5; on grids filled with SrTiO3 it was 0.1-0.9 %
-// further off with FP32 sums and phases reduced to [0, 1)). 64 instead of 32 registers of sums and half the FMA rate cost 27 us
-// on 66 at 2048^2 with 10 jobs of 1024 atoms, 4.6 % of a build.  Slower still: weights read from global
-// memory by every thread (+20 us), a thread per real component, half the registers and twice the
-// threads (+42 us), E loaded eight groups ahead (126 registers, +12 us).
+// further off with FP32 sums and phases reduced to [0, 1)).  64 instead of 32 registers of sums and half
+// the FMA rate cost 27 us on 66 at 2048^2 with 10 jobs of 1024 atoms, 4.6 % of a build.  Slower still:
+// weights read from global memory by every thread (+20 us), a thread per real component, half the
+// registers and twice the threads (+42 us), E loaded eight groups ahead (126 registers, +12 us).
 // PIECES: of the groups only [g0, g0 + ex_rows) are held.  The sums go on from one piece to the next in
 // fine64, in the same order (the groups that wrap around sort last), so the pieces change no bit.
 template <bool PIECES>
